@@ -140,7 +140,8 @@ typedef enum {
 
 /* Arithmetic of the FP64 merge-path kernel. */
 typedef enum {
-  SpB_VNEC_ARITH_AUTO = 0, /* DF32 when A's values allow it, else FP64 */
+  SpB_VNEC_ARITH_AUTO = 0, /* FP64 in the tile kernel (the default); in the pipelined one
+                              DF32 when A's values allow it, else FP64 */
   SpB_VNEC_ARITH_FP64 = 1, /* one FP64 FMA per nonzero */
   SpB_VNEC_ARITH_DF32 = 2  /* double-float on the FP32 pipe: products and sums
                               with ~2^-46 relative error, needs |a|,|x| in
@@ -153,7 +154,9 @@ typedef struct {
   int items_per_thread;  /* 0: default; sliced plans: load steps in flight 4/8/12/16,
                             0 or -1: each timed on the matrix at plan build (y is
                             the same at every value) */
-  int pipeline_stages;   /* merge-path: 0 default (2), 1 unpipelined kernel, 2-3 stages */
+  int pipeline_stages;   /* merge-path: 1 the tile kernel, 2-3 stages of the pipelined one; 0: the
+                            tile kernel, except FP64 plans below 2^26 nonzeros that ask for DF32
+                            sums or a tile shape other than 256 x 7 (pipelined, 2 stages) */
   int arithmetic;        /* SpB_VNEC_arith_ext (FP64 values) */
   int window_rows;       /* sliced: rows sorted within windows of this size (0: 65536) */
   int long_row_len;      /* sliced: rows longer than this are chunked (0: 1024) */

@@ -136,8 +136,6 @@ bool mp_partition(const MpMatrix& m, cudaStream_t s);
 // between the tile and fix-up kernels, and after the fix-up kernel.
 bool mp_spmv(const MpMatrix& m, MpForm form, const void* x, void* y, cudaStream_t s,
              cudaEvent_t* events = nullptr);
-// Dynamic shared memory bytes of one tile for a shape and value size.
-size_t mp_smem_bytes(const MpShape& sh, size_t value_bytes);
 // Kernel launches per mp_spmv call.
 constexpr int kMpLaunchesPerCall = 2;
 

@@ -453,22 +453,25 @@ std::unique_ptr<Plan> build_merge_path(const CsrView& v, const SpB_VNEC_options_
   const bool wide = (v.n_rows + v.nnz) >= ((int64_t)1 << 31) - 1 || (opts && opts->offsets64 > 0);
   const int req_stages = opts ? opts->pipeline_stages : 0;
   const int req_arith = opts ? opts->arithmetic : SpB_VNEC_ARITH_AUTO;
-  // The pipelined kernel serves FP64 matrices with int32 merge coordinates.
-  // By default large matrices (>= 2^26 nonzeros) take the unpipelined kernel
-  // with 256 x 4 tiles: on GB300 timings of matrices that size it is 1.5x
-  // faster (more resident warps than the shared-memory pipeline allows).
+  // The tile kernel (mp_kernels.cu) runs every plan that does not ask for the
+  // pipelined one (FP64 values, int32 merge coordinates, below 2^26 nonzeros
+  // by default): by two or more stages, by DF32 sums, or by a tile shape other
+  // than 256 x 7, which only the pipelined kernel takes when no stage count is
+  // given.  The tile kernel is 2 to 3x faster on every matrix family, from 10^5
+  // nonzeros (R-MAT 2^14: 17.6 -> 12.5 us) to 5 10^7 (2^22: 874 -> 293), and
+  // sums in FP64 where the pipelined default took double-float pairs.
   constexpr int64_t kPipelineMaxNnz = (int64_t)1 << 26;
   const bool large = req_stages == 0 && v.nnz >= kPipelineMaxNnz;
-  p->pipelined = v.type == SpB_FP64 && !wide && req_stages != 1 && !large;
   MpShape sh;
-  if (p->pipelined) {
-    sh.tpb = 256;
-    sh.ipt = 7;
-  } else if (large) {
-    sh.ipt = 4;
-  }
+  const bool other_shape = opts && ((opts->threads_per_block && opts->threads_per_block != sh.tpb) ||
+                                    (opts->items_per_thread && opts->items_per_thread != sh.ipt));
+  p->pipelined = v.type == SpB_FP64 && !wide && req_stages != 1 && !large &&
+                 (req_stages >= 2 || req_arith == SpB_VNEC_ARITH_DF32 || other_shape);
   if (opts && opts->threads_per_block) sh.tpb = opts->threads_per_block;
   if (opts && opts->items_per_thread) sh.ipt = opts->items_per_thread;
+  // The default tile: small CTAs overlap the phases of a tile best (against
+  // 256 x 7: R-MAT 2^22 361 -> 293 us, 27-point stencil 120^3 234 -> 172).
+  if (!p->pipelined && !(opts && (opts->threads_per_block || opts->items_per_thread))) sh.tpb = 128;
   const int stages = req_stages >= 2 ? req_stages : 2;
   if (p->pipelined ? mp2_smem(sh.tpb, sh.ipt, stages) == 0 : !shape_supported(sh.tpb, sh.ipt)) {
     set_error(p->pipelined ? "unsupported pipelined tile shape (256x7 s2/s3, 256x12 s2, 128x12 s3, 512x5 s2)"

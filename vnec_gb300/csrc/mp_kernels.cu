@@ -4,16 +4,21 @@
 //
 // Work decomposition.  The merge of the row-end list (row_ptr[1..n]) and the
 // nonzero counting list (0..nnz-1) has n_rows + nnz items.  It is cut into
-// tiles of TPB*IPT items, one CTA per tile; the tile boundaries are found once
-// per matrix (plan time) by mp_partition_kernel.  Inside a tile:
-//   1. stage: the tile's values, the gathered x[col] and its row ends are
-//      copied to shared memory with coalesced loads (values and columns are
-//      read once, so they are loaded with the streaming cache hint; x is
-//      gathered through the read-only path so it stays resident in L2);
-//   2. consume: each thread runs the merge path over IPT consecutive items of
-//      the tile — one FMA per nonzero, a row result at each row end — exactly
-//      the per-thread loop of the reference's OpenMP threads, at warp lane
-//      granularity;
+// tiles of a fixed number of items, one CTA per tile; the tile boundaries are
+// found once per matrix (plan time) by mp_partition_kernel, so a tile holds a
+// bounded number of rows and of nonzeros whatever the row lengths.  Inside a
+// tile:
+//   1. every thread owns 8 consecutive nonzeros, cut at multiples of 8 of the
+//      nonzero index: columns and values come in with 32-byte vector loads
+//      (read once, no L1 allocation) straight into registers, and the 8
+//      gathers of x are in flight together;
+//   2. the tile's row ends are read once, coalesced, and each row with a
+//      nonzero in the tile writes its number to a 16-bit slot at its last
+//      nonzero's place; a row with none is stored as zero right away.  A
+//      thread then finds the row ends among its 8 nonzeros with one 16-byte
+//      shared-memory read: no search and no merge walk, and the only FP64
+//      work per nonzero is its FMA (an FP64 operation takes the pipe of a
+//      whole warp for 16 cycles here, whichever lanes need it);
 //   3. carry: a thread whose segment starts inside a row adds the partial sums
 //      of the preceding threads that stopped in the same row, found by a
 //      segmented scan over the threads (warp shuffles plus one scan over the
@@ -22,12 +27,16 @@
 //   4. fix-up (second, tiny launch): rows spanning tiles receive the ordered
 //      sum of the carries of the tiles that stopped inside them — the
 //      counterpart of the reference's serial carry loop (:159-164).
-// The FP64 form performs exactly one FP64 FMA per nonzero plus at most
-// log2(32) + log2(warps) adds per thread for the carries: on GB300 the FP64
-// pipe (about 0.6 T FMA/s) is close to the HBM rate for SpMV, so no other
-// FP64 work is done in the loop.  (A walk back over the preceding threads'
-// partials costs one add per thread a row spans, quadratic in the rows that
-// cover a whole tile: on R-MAT 2^24 it kept the FP64 pipe 70% busy.)
+//
+// What bounds it: the x gathers' L1/L2 requests on power-law columns, as in
+// the sliced kernel, without its hot-column window.
+// Measured on GB300 (R-MAT 2^22, 49 M nonzeros; 27-point stencil 120^3; us a
+// call, against the kernels it replaced as the default: pipelined DF32 tiles,
+// whose shared-memory merge walk bound them): FP64 874 -> 293 and 455 -> 172;
+// the FP32 type 193 and 102.  FP64 pipe 60% busy, L1 65%, L2 53 to 68%: no one
+// unit binds, the phases of a tile do.  Small CTAs overlap them best: tiles of
+// 128 x 7 items (one thread per 8 places) against 256 x 7 are 7 to 20% faster,
+// 16 nonzeros a thread up to 15% slower on power-law rows.
 
 #include <cuda_runtime.h>
 
@@ -41,7 +50,6 @@ namespace vnec {
 namespace {
 
 template <typename T> __device__ __forceinline__ T ld_stream(const T* p) { return __ldcs(p); }
-__device__ __forceinline__ long long ld_stream(const long long* p) { return __ldcs(p); }
 
 template <typename V> __device__ __forceinline__ V fma_v(V a, V b, V c);
 template <> __device__ __forceinline__ double fma_v<double>(double a, double b, double c) { return fma(a, b, c); }
@@ -76,164 +84,256 @@ __global__ void mp_partition_kernel(const Off* __restrict__ row_end, Off n_rows,
   tile_nz[t] = diag - r;
 }
 
-// One CTA per tile.  Shared memory: s_val[IPC], s_x[IPC] (V), s_end[IPC]
-// (int, row ends relative to the tile's first nonzero), per-warp carry
-// totals, open flags and carry-ins (TPB / 32 each).
-template <typename V, typename Off, int TPB, int IPT>
-__global__ void __launch_bounds__(TPB)
+// N (a multiple of 8) consecutive items as 32-byte vectors; `p` is aligned to
+// 32 bytes.
+template <int N> __device__ __forceinline__ void load_items(const double* p, double (&v)[N]) {
+#pragma unroll
+  for (int h = 0; h < N; h += 4)
+    asm("ld.global.nc.L1::no_allocate.v4.f64 {%0, %1, %2, %3}, [%4];"
+        : "=d"(v[h]), "=d"(v[h + 1]), "=d"(v[h + 2]), "=d"(v[h + 3])
+        : "l"(p + h));
+}
+template <int N> __device__ __forceinline__ void load_items(const float* p, float (&v)[N]) {
+#pragma unroll
+  for (int h = 0; h < N; h += 8)
+    asm("ld.global.nc.L1::no_allocate.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=f"(v[h]), "=f"(v[h + 1]), "=f"(v[h + 2]), "=f"(v[h + 3]), "=f"(v[h + 4]), "=f"(v[h + 5]),
+          "=f"(v[h + 6]), "=f"(v[h + 7])
+        : "l"(p + h));
+}
+template <int N> __device__ __forceinline__ void load_items(const int32_t* p, int32_t (&v)[N]) {
+#pragma unroll
+  for (int h = 0; h < N; h += 8)
+    asm("ld.global.nc.L1::no_allocate.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=r"(v[h]), "=r"(v[h + 1]), "=r"(v[h + 2]), "=r"(v[h + 3]), "=r"(v[h + 4]), "=r"(v[h + 5]),
+          "=r"(v[h + 6]), "=r"(v[h + 7])
+        : "l"(p + h));
+}
+
+constexpr unsigned kNoRow = 0xffffu;  // slot of a nonzero that ends no row
+constexpr int E = 8;                  // nonzeros per thread
+
+// Threads of a tile of `items` merge items: E nonzeros each, and one thread
+// more because the tile's first nonzero may lie inside its thread's E.
+constexpr int tile_threads(int items) { return ((items + E - 1) / E + 1 + 31) / 32 * 32; }
+constexpr int kMaxTileThreads = tile_threads(256 * 10);
+
+// One CTA per tile, of at most T threads with E nonzeros each; at least B CTAs
+// fit an SM.  Dynamic shared memory: a 16-bit slot per nonzero place, then each thread's head and tail sums.  `vec`: col and val
+// are 32-byte aligned.
+template <typename V, typename Off, int T, int B>
+__global__ void __launch_bounds__(T, B)
 mp_spmv_kernel(const Off* __restrict__ row_end, const int32_t* __restrict__ col, const V* __restrict__ val,
                const V* __restrict__ x, V* __restrict__ y, const Off* __restrict__ tile_row,
-               const Off* __restrict__ tile_nz, Off* __restrict__ carry_row, V* __restrict__ carry_val) {
-  constexpr int IPC = TPB * IPT;
-  constexpr int kW = TPB / 32;
+               const Off* __restrict__ tile_nz, Off nnz, bool vec, Off* __restrict__ carry_row,
+               V* __restrict__ carry_val) {
   constexpr unsigned kFull = 0xffffffffu;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  V* s_val = reinterpret_cast<V*>(smem_raw);
-  V* s_x = s_val + IPC;
-  V* w_run = s_x + IPC;  // [kW] warp totals of the open run
-  V* w_cin = w_run + kW;  // [kW] carry into each warp
-  int* s_end = reinterpret_cast<int*>(w_cin + kW);
-  int* w_open = s_end + IPC;  // [kW]
-
+  extern __shared__ uint4 s_slots[];
+  V* const s_tail = reinterpret_cast<V*>(s_slots + (E / 8) * blockDim.x);
+  V* const s_head = s_tail + blockDim.x;
   const int tile = blockIdx.x;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int tid = threadIdx.x, lane = tid & 31;
   const Off x0 = tile_row[tile], y0 = tile_nz[tile];
   const Off x1 = tile_row[tile + 1], y1 = tile_nz[tile + 1];
   const int nrows = (int)(x1 - x0);
-  const int nnz = (int)(y1 - y0);
+  const int lead = (int)(y0 & (E - 1));   // places before the tile's first nonzero
+  const int end = lead + (int)(y1 - y0);  // one past its last
+  const Off origin = y0 - lead;           // nonzero at place 0, a multiple of E
+  const int q = E * tid;                  // this thread's first place
 
-  // 1. stage values, gathered x and row ends.
+  // 1. columns and values, then x.  Places outside the tile hold value and x 0.
+  V v[E], xv[E];
   {
-    const int32_t* c_t = col + y0;
-    const V* v_t = val + y0;
-#pragma unroll 4
-    for (int i = tid; i < nnz; i += TPB) {
-      int c = ld_stream(c_t + i);
-      s_val[i] = ld_stream(v_t + i);
-      s_x[i] = __ldg(x + c);
-    }
-    const Off* e_t = row_end + x0;
-    for (int i = tid; i < nrows; i += TPB) s_end[i] = (int)(ld_stream(e_t + i) - y0);
-  }
-  __syncthreads();
-
-  // 2. per-thread merge path over IPT items.
-  const int total = nrows + nnz;
-  const int d = min(tid * IPT, total);
-  int rr = merge_search<int>(s_end, d, nrows, nnz);
-  int kk = d - rr;
-  const int dend = min(d + IPT, total);
-  V acc = V(0);
-  V first_val = V(0);
-  int first = -1;
+    const int32_t* cp = col + origin + q;
+    const V* vp = val + origin + q;
+    int32_t c[E];
+    if (vec && q < end && nnz - origin >= q + E) {
+      load_items<E>(cp, c);
+      load_items<E>(vp, v);
 #pragma unroll
-  for (int it = 0; it < IPT; ++it) {
-    if (d + it < dend) {
-      if (rr < nrows && s_end[rr] <= kk) {
-        if (first < 0) {
-          first = rr;
-          first_val = acc;
-        } else {
-          y[x0 + rr] = acc;
-        }
-        acc = V(0);
-        ++rr;
-      } else {
-        acc = fma_v<V>(s_val[kk], s_x[kk], acc);
-        ++kk;
+      for (int j = 0; j < E; ++j) {
+        const bool in = q + j >= lead && q + j < end;
+        xv[j] = in ? __ldg(x + c[j]) : V(0);
+        if (!in) v[j] = V(0);
+      }
+    } else {
+#pragma unroll
+      for (int j = 0; j < E; ++j) {
+        const bool in = q + j >= lead && q + j < end;
+        c[j] = in ? ld_stream(cp + j) : 0;
+        v[j] = in ? ld_stream(vp + j) : V(0);
+        xv[j] = in ? __ldg(x + c[j]) : V(0);
       }
     }
   }
 
-  // 3. in-tile carries.  A thread that emitted a row starts a new run with its
-  // tail partial; a thread that did not is still inside the row of the
-  // threads before it.  A segmented inclusive scan over the threads (warp
-  // shuffles, then one scan over the warp totals) gives every thread the sum
-  // of the open run before it in log steps, however many threads a row spans.
-  V run = acc;
-  int open = first < 0;
-  for (int dist = 1; dist < 32; dist <<= 1) {
-    if (!__ballot_sync(kFull, open && lane >= dist)) break;
-    const V up = __shfl_up_sync(kFull, run, dist);
-    const int up_open = __shfl_up_sync(kFull, open, dist);
-    if (open && lane >= dist) {
-      run += up;
-      open = up_open;
+  // 2. row ends: row r of the tile ends after the nonzero at place e - 1; its
+  // first nonzero in the tile is at the end of the row before it.
+#pragma unroll
+  for (int h = 0; h < E / 8; ++h) s_slots[(E / 8) * tid + h] = make_uint4(~0u, ~0u, ~0u, ~0u);
+  __syncthreads();
+  {
+    unsigned short* slot = reinterpret_cast<unsigned short*>(s_slots);
+    for (int r = tid; r < nrows; r += blockDim.x) {
+      const Off e = row_end[x0 + r], b = r ? row_end[x0 + r - 1] : y0;
+      if (e > b)
+        slot[(int)(e - y0) + lead - 1] = (unsigned short)r;
+      else
+        y[x0 + r] = V(0);
     }
   }
-  if (lane == 31) {
-    w_run[warp] = run;
-    w_open[warp] = open;
-  }
   __syncthreads();
-  if (warp == 0) {
-    V cv = lane < kW ? w_run[lane] : V(0);
-    int co = lane < kW ? w_open[lane] : 0;
-    for (int dist = 1; dist < kW; dist <<= 1) {
-      const V up = __shfl_up_sync(kFull, cv, dist);
-      const int up_open = __shfl_up_sync(kFull, co, dist);
-      if (co && lane >= dist) {
-        cv += up;
-        co = up_open;
-      }
+  unsigned sw[E / 2];
+#pragma unroll
+  for (int h = 0; h < E / 8; ++h) {
+    const uint4 s4 = s_slots[(E / 8) * tid + h];
+    sw[4 * h] = s4.x;
+    sw[4 * h + 1] = s4.y;
+    sw[4 * h + 2] = s4.z;
+    sw[4 * h + 3] = s4.w;
+  }
+  // The sum up to the thread's first row end goes to its head, what follows
+  // its last row end (everything, if no row ends here) to its tail; a row
+  // between two ends is complete.
+  V acc = V(0);
+  bool any = false;
+#pragma unroll
+  for (int j = 0; j < E; ++j) {
+    acc = fma_v<V>(v[j], xv[j], acc);  // outside the branch: one FP64 instruction for the whole warp
+    const unsigned r = (sw[j >> 1] >> (16 * (j & 1))) & 0xffffu;
+    if (r != kNoRow) {
+      if (any)
+        y[x0 + r] = acc;
+      else
+        s_head[tid] = acc;
+      any = true;
+      acc = V(0);
     }
-    const V ex = __shfl_up_sync(kFull, cv, 1);
-    if (lane < kW) w_cin[lane] = lane == 0 ? V(0) : ex;
   }
+  s_tail[tid] = acc;
   __syncthreads();
-  const V prev = __shfl_up_sync(kFull, run, 1);
-  const int prev_open = __shfl_up_sync(kFull, open, 1);
-  if (first >= 0) {
-    V cin;
-    if (lane == 0)
-      cin = w_cin[warp];
-    else
-      cin = prev_open ? prev + w_cin[warp] : prev;
-    y[x0 + first] = first_val + cin;
-  }
-  if (tid == TPB - 1) {
-    carry_row[tile] = x1;
-    carry_val[tile] = open ? run + w_cin[warp] : run;
+
+  // 3. rows that begin in an earlier thread than they end in, or at its edge:
+  // lane r adds the tails from the row's first thread on, then the head of its
+  // last.  Where that takes fewer FP64 instructions of the warp (the longest
+  // walk against kShare for each row past kWalk threads), the lanes share the
+  // longer rows instead.  "Row" nrows is what the tile leaves open: the carry.
+  constexpr int kWalk = 4, kShare = 6;
+  for (int r0 = tid - lane; r0 <= nrows; r0 += blockDim.x) {
+    const int r = r0 + lane;
+    int b = 0, e = 0;
+    bool mine = false;
+    if (r <= nrows) {
+      e = r < nrows ? (int)(row_end[x0 + r] - y0) + lead : end;
+      b = r ? (int)(row_end[x0 + r - 1] - y0) + lead : lead;
+      mine = e > b;
+      if (b == lead) b = 0;  // the zero places before the tile count as the first row's
+      mine = mine && (r == nrows || b <= (e - 1) / E * E);
+    }
+    const int te = (e - 1) / E, t0 = b / E, t1 = r < nrows ? te : te + 1;  // tails t0 .. t1 - 1
+    const int span = mine ? t1 - t0 : 0;
+    const unsigned many = __ballot_sync(kFull, span > kWalk);
+    const int longest = (int)__reduce_max_sync(kFull, (unsigned)span);  // every lane takes part
+    const bool shared = span > kWalk && kWalk + kShare * __popc(many) < longest;
+    V s = V(0);
+    if (mine && !shared)
+      for (int t = t0; t < t1; ++t) s += s_tail[t];
+    for (unsigned m = __ballot_sync(kFull, shared); m; m &= m - 1) {
+      const int src = __ffs(m) - 1;
+      const int u0 = __shfl_sync(kFull, t0, src), u1 = __shfl_sync(kFull, t1, src);
+      V p = V(0);
+      for (int t = u0 + lane; t < u1; t += 32) p += s_tail[t];
+      for (int off = 16; off > 0; off >>= 1) p += __shfl_xor_sync(kFull, p, off);
+      if (lane == src) s = p;
+    }
+    if (r < nrows) {
+      if (mine) y[x0 + r] = t1 > t0 ? s + s_head[te] : s_head[te];
+    } else if (r == nrows) {
+      carry_row[tile] = x1;
+      carry_val[tile] = s;
+    }
   }
 }
 
 // 4. cross-tile carries: the first tile of each run of tiles that stopped in
-// the same row adds the run's carries, in tile order, to that row.
+// the same row adds the run's carries to that row.  A run of up to four tiles
+// is summed by its thread; a longer one (a row of many tiles) by the thread's
+// warp, lane l taking tiles l, l + 32, ... of the run, joined by a fixed xor
+// tree, so a hub row costs a few loads in a row instead of one per tile.
 template <typename V, typename Off>
 __global__ void mp_fixup_kernel(const Off* __restrict__ carry_row, const V* __restrict__ carry_val,
                                 long long num_tiles, Off n_rows, V* __restrict__ y) {
-  long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (t >= num_tiles) return;
-  Off r = carry_row[t];
-  if (r >= n_rows) return;
-  if (t > 0 && carry_row[t - 1] == r) return;
-  V s = V(0);
-  for (long long u = t; u < num_tiles && carry_row[u] == r; ++u) s += carry_val[u];
-  y[r] += s;
+  constexpr unsigned kFull = 0xffffffffu;
+  constexpr int kShort = 4;
+  const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  const int lane = threadIdx.x & 31;
+  Off r = n_rows;
+  bool head = false, longer = false;
+  if (t < num_tiles) {
+    r = carry_row[t];
+    head = r < n_rows && (t == 0 || carry_row[t - 1] != r);
+    longer = head && t + kShort < num_tiles && carry_row[t + kShort] == r;
+  }
+  if (head && !longer) {
+    V s = V(0);
+#pragma unroll
+    for (int u = 0; u < kShort; ++u)
+      if (t + u < num_tiles && carry_row[t + u] == r) s += carry_val[t + u];
+    y[r] += s;
+  }
+  for (unsigned m = __ballot_sync(kFull, longer); m; m &= m - 1) {
+    const int src = __ffs(m) - 1;
+    const long long t0 = t - lane + src;
+    const Off row = __shfl_sync(kFull, r, src);
+    V s = V(0);
+    for (long long u = t0 + lane;; u += 32) {
+      const bool in = u < num_tiles && carry_row[u] == row;
+      if (in) s += carry_val[u];
+      if (!__all_sync(kFull, in)) break;  // the run is contiguous: it ends here
+    }
+    for (int off = 16; off > 0; off >>= 1) s += __shfl_xor_sync(kFull, s, off);
+    if (lane == 0) y[row] += s;
+  }
 }
 
-template <typename V, typename Off, int TPB, int IPT>
-bool launch_mp(const MpMatrix& m, const void* x, void* y, cudaStream_t s, cudaEvent_t* ev) {
-  auto kern = mp_spmv_kernel<V, Off, TPB, IPT>;
-  MpShape sh;
-  sh.tpb = TPB;
-  sh.ipt = IPT;
-  size_t smem = mp_smem_bytes(sh, sizeof(V));
+template <typename V, typename Off, int T, int B>
+bool launch_tiles(const MpMatrix& m, int threads, const void* x, void* y, cudaStream_t s) {
+  auto kern = mp_spmv_kernel<V, Off, T, B>;
+  // A few KB of shared memory per CTA: leave the rest of the array to L1, which
+  // serves the x gathers.
   static std::atomic<unsigned long long> configured{0};  // per instantiation, per device
   if (!once_per_device(configured, [&] {
-        return VNEC_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        return VNEC_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 32));
       }))
     return false;
   if (m.num_tiles > 0x7fffffffLL) {
     set_error("merge-path: tile count exceeds the grid limit");
     return false;
   }
-  if (ev && !VNEC_CUDA(cudaEventRecord(ev[0], s))) return false;
-  kern<<<(unsigned)m.num_tiles, TPB, smem, s>>>(
+  const bool vec = ((reinterpret_cast<uintptr_t>(m.col) | reinterpret_cast<uintptr_t>(m.val)) & 31) == 0;
+  kern<<<(unsigned)m.num_tiles, threads, (size_t)threads * (E * sizeof(unsigned short) + 2 * sizeof(V)), s>>>(
       static_cast<const Off*>(m.row_end), m.col, static_cast<const V*>(m.val), static_cast<const V*>(x),
-      static_cast<V*>(y), static_cast<const Off*>(m.tile_row), static_cast<const Off*>(m.tile_nz),
+      static_cast<V*>(y), static_cast<const Off*>(m.tile_row), static_cast<const Off*>(m.tile_nz), (Off)m.nnz, vec,
       static_cast<Off*>(m.carry_row), static_cast<V*>(m.carry_val));
-  if (!VNEC_CUDA(cudaGetLastError())) return false;
+  return VNEC_CUDA(cudaGetLastError());
+}
+
+template <typename V, typename Off>
+bool launch_mp(const MpMatrix& m, const void* x, void* y, cudaStream_t s, cudaEvent_t* ev) {
+  if (ev && !VNEC_CUDA(cudaEventRecord(ev[0], s))) return false;
+  const int threads = tile_threads((int)m.shape.items_per_tile());
+  if (threads > kMaxTileThreads) {
+    set_error("merge-path: unsupported tile shape");
+    return false;
+  }
+  // 40 warps of an SM for FP64 (48 registers a thread), 64 for FP32: FP64 runs
+  // at 40 as at 48 (40 registers, which spill) or at 36, FP32 slows down by 7%
+  // at 48 warps and by 15% at 40 (R-MAT 2^22: 193, 207 and 225 us).
+  constexpr int kB = sizeof(V) == 8 ? 10 : 16;
+  if (!(threads <= 128   ? launch_tiles<V, Off, 128, kB>(m, threads, x, y, s)
+        : threads <= 256 ? launch_tiles<V, Off, 256, kB / 2>(m, threads, x, y, s)
+                         : launch_tiles<V, Off, kMaxTileThreads, 1>(m, threads, x, y, s)))
+    return false;
   if (ev && !VNEC_CUDA(cudaEventRecord(ev[1], s))) return false;
   const int fb = 256;
   long long fg = (m.num_tiles + fb - 1) / fb;
@@ -245,28 +345,7 @@ bool launch_mp(const MpMatrix& m, const void* x, void* y, cudaStream_t s, cudaEv
   return true;
 }
 
-template <typename V, typename Off>
-bool dispatch_shape(const MpMatrix& m, const void* x, void* y, cudaStream_t s, cudaEvent_t* ev) {
-  const int tpb = m.shape.tpb, ipt = m.shape.ipt;
-#define VNEC_MP_CASE(T, I) \
-  if (tpb == T && ipt == I) return launch_mp<V, Off, T, I>(m, x, y, s, ev);
-  VNEC_MP_CASE(128, 4)
-  VNEC_MP_CASE(128, 7)
-  VNEC_MP_CASE(128, 10)
-  VNEC_MP_CASE(256, 4)
-  VNEC_MP_CASE(256, 7)
-  VNEC_MP_CASE(256, 10)
-#undef VNEC_MP_CASE
-  set_error("merge-path: unsupported tile shape");
-  return false;
-}
-
 }  // namespace
-
-size_t mp_smem_bytes(const MpShape& sh, size_t value_bytes) {
-  const size_t ipc = (size_t)sh.tpb * sh.ipt, warps = (size_t)sh.tpb / 32;
-  return 2 * ipc * value_bytes + 2 * warps * value_bytes + ipc * sizeof(int) + warps * sizeof(int);
-}
 
 bool mp_partition(const MpMatrix& m, cudaStream_t s) {
   long long ipc = m.shape.items_per_tile();
@@ -288,9 +367,9 @@ bool mp_spmv(const MpMatrix& m, MpForm form, const void* x, void* y, cudaStream_
   if (m.n_rows == 0) return true;
   switch (form) {
     case MpForm::kF64:
-      return m.wide ? dispatch_shape<double, long long>(m, x, y, s, ev) : dispatch_shape<double, int>(m, x, y, s, ev);
+      return m.wide ? launch_mp<double, long long>(m, x, y, s, ev) : launch_mp<double, int>(m, x, y, s, ev);
     case MpForm::kF32:
-      return m.wide ? dispatch_shape<float, long long>(m, x, y, s, ev) : dispatch_shape<float, int>(m, x, y, s, ev);
+      return m.wide ? launch_mp<float, long long>(m, x, y, s, ev) : launch_mp<float, int>(m, x, y, s, ev);
   }
   set_error("merge-path: unknown value form");
   return false;

@@ -17,8 +17,9 @@
 namespace vnec {
 namespace {
 
-// Merge-path configurations: (items per thread, pipeline stages) with 256
-// threads; ipt 4 runs the unpipelined kernel.  Warp-task configurations:
+// Merge-path configurations by items per thread: 4 and 7 run the tile kernel
+// (256 x 4, and 128 x 7, the tile of a default L plan), 12 the pipelined kernel
+// with 256 threads and two stages.  Warp-task configurations:
 // long-row chunk x dense-block fill threshold (1: every row with a block goes
 // dense, 1001: every row sliced).
 const TuneConfig kConfigs[kNumConfigs] = {
@@ -100,9 +101,9 @@ SpB_VNEC_options_ext config_options(int i, const SpB_VNEC_options_ext* base) {
   const TuneConfig& c = kConfigs[i];
   o.kernel = c.kernel;
   if (c.kernel == SpB_VNEC_KERNEL_L) {
-    o.threads_per_block = 256;
+    o.threads_per_block = c.chunk == 7 ? 128 : 256;
     o.items_per_thread = c.chunk;
-    o.pipeline_stages = c.chunk == 4 ? 1 : 2;
+    o.pipeline_stages = c.chunk == 12 ? 2 : 1;
   } else {
     o.threads_per_block = 0;
     o.items_per_thread = -1;  // sliced parts time their unroll on the matrix
@@ -156,8 +157,8 @@ int autotune_search(const CsrView& v, const SpB_VNEC_options_ext* base, int reps
 // VNEC-S — here the merge path, the pure dense-block configuration and the
 // pure sliced configuration with their default chunk.
 int rule_choice(const CsrView& v) {
-  // VNEC-L: the merge-path configuration a default L plan takes at this size.
-  if (v.n_rows >= 3000000) return v.nnz >= ((int64_t)1 << 26) ? 0 : 1;
+  // VNEC-L: the merge-path configuration a default L plan takes.
+  if (v.n_rows >= 3000000) return 1;
   const IrdParams prm = ird_params(v.type);
   const float ird = ird_ratio(v, prm);
   const bool dense = ird >= prm.threshold && cols_sorted(v);
