@@ -34,6 +34,7 @@
 #include "batch.h"
 #include "common.h"
 #include "df32.cuh"
+#include "launch.cuh"
 
 namespace vnec {
 namespace {
@@ -303,11 +304,15 @@ __device__ __forceinline__ void run_tasks(const BatchArgs& a, const typename Cd:
 
 template <class Cd, int R, int U, bool STAGED>
 __global__ void __launch_bounds__(256) batch_kernel(const BatchArgs a) {
+  release_next();
+  wait_for_previous();
   run_tasks<Cd, R, U, STAGED>(a, static_cast<const typename Cd::X*>(a.x));
 }
 
 template <int R, int U, bool STAGED>
 __global__ void __launch_bounds__(256) batch_df32_kernel(const BatchArgs a) {
+  release_next();
+  wait_for_previous();
   if (*reinterpret_cast<const volatile int*>(a.flag))
     run_tasks<CodecDF32Guard, R, U, STAGED>(a, a.x64);
   else
@@ -318,21 +323,22 @@ __global__ void __launch_bounds__(256) batch_df32_kernel(const BatchArgs a) {
 // stages the entries in registers (STAGED) with the mode-0 step count.
 template <int R, int MODE> constexpr int unroll_for() { return (R >= 4 ? 2 : 8 / R) * (MODE == 1 ? 2 : 1); }
 
-template <int R, int MODE> void* kernel_for(int precision) {
+using BatchKernel = void (*)(BatchArgs);
+template <int R, int MODE> BatchKernel kernel_for(int precision) {
   constexpr int U = unroll_for<R, MODE>();
   constexpr bool ST = MODE == 2;
   switch (precision) {
-    case kPrecFP32: return reinterpret_cast<void*>(&batch_kernel<CodecF32, R, U, ST>);
-    case kPrecDF32: return reinterpret_cast<void*>(&batch_df32_kernel<R, U, ST>);
-    default: return reinterpret_cast<void*>(&batch_kernel<CodecF64, R, U, ST>);
+    case kPrecFP32: return &batch_kernel<CodecF32, R, U, ST>;
+    case kPrecDF32: return &batch_df32_kernel<R, U, ST>;
+    default: return &batch_kernel<CodecF64, R, U, ST>;
   }
 }
 
-template <int R> void* kernel_for_mode(int precision, int mode) {
+template <int R> BatchKernel kernel_for_mode(int precision, int mode) {
   return mode == 2 ? kernel_for<R, 2>(precision) : mode == 1 ? kernel_for<R, 1>(precision) : kernel_for<R, 0>(precision);
 }
 
-void* pick_kernel(int precision, int r, int mode) {
+BatchKernel pick_kernel(int precision, int r, int mode) {
   switch (r) {
     case 1: return kernel_for_mode<1>(precision, mode);
     case 2: return kernel_for_mode<2>(precision, mode);
@@ -351,7 +357,7 @@ int log2i(int v) {
 }  // namespace
 
 int batch_grid(int precision, int rhs_per_lane, int warps_per_block, int mode) {
-  void* fn = pick_kernel(precision, rhs_per_lane, mode);
+  const BatchKernel fn = pick_kernel(precision, rhs_per_lane, mode);
   if (!fn || (warps_per_block != 4 && warps_per_block != 8)) return 0;
   int dev = 0, sms = 0, per_sm = 0;
   if (!VNEC_CUDA(cudaGetDevice(&dev)) ||
@@ -400,7 +406,7 @@ bool batch_spmm_range(const BatchMatrix& m, const double* X, double* Y, cudaStre
   a.y = Y;
   a.klog2 = log2i(m.k);
   a.llog2 = log2i(m.lanes);
-  void* fn = pick_kernel(m.precision, R, m.mode);
+  const BatchKernel fn = pick_kernel(m.precision, R, m.mode);
   // Persistent warps stride the task list; with per_task every warp takes one
   // task and the hardware dispatches the blocks in task order, so the tasks in
   // flight stay a compact window of the list (and of X's rows).
@@ -411,8 +417,7 @@ bool batch_spmm_range(const BatchMatrix& m, const double* X, double* Y, cudaStre
   }
   const int grid = m.per_task ? (int)per_task_grid
                               : (int)std::min<long long>(m.grid, std::max<long long>(1, (a.num_tasks + 7) / 8));
-  void* args[] = {&a};
-  return VNEC_CUDA(cudaLaunchKernel(fn, dim3((unsigned)grid), dim3((unsigned)(m.warps_per_block * 32)), args, 0, s));
+  return launch_chained(fn, (unsigned)grid, (unsigned)(m.warps_per_block * 32), 0, s, a);
 }
 
 }  // namespace vnec

@@ -127,6 +127,9 @@ struct MpMatrix {
   void* carry_val = nullptr;       // num_tiles scratch
   int64_t num_tiles = 0;
   MpShape shape;
+  // The arrays above (scratch aside) were in place before the call: a plan's,
+  // not a caller's that an earlier launch on the stream may still be writing.
+  bool in_place = false;
 };
 
 // Fills tile_row / tile_nz (device) for the given shape.

@@ -491,6 +491,7 @@ std::unique_ptr<Plan> build_merge_path(const CsrView& v, const SpB_VNEC_options_
   m.nnz = v.nnz;
   m.shape = sh;
   m.wide = wide;
+  m.in_place = true;
   const size_t ob = m.wide ? 8 : 4;
   const size_t vb = v.value_bytes();
   const int64_t ipc = sh.items_per_tile();

@@ -44,6 +44,7 @@
 #include <mutex>
 
 #include "common.h"
+#include "launch.cuh"
 #include "vnec_gb300.h"
 
 namespace vnec {
@@ -133,6 +134,7 @@ mp_spmv_kernel(const Off* __restrict__ row_end, const int32_t* __restrict__ col,
   V* const s_head = s_tail + blockDim.x;
   const int tile = blockIdx.x;
   const int tid = threadIdx.x, lane = tid & 31;
+  release_next();
   const Off x0 = tile_row[tile], y0 = tile_nz[tile];
   const Off x1 = tile_row[tile + 1], y1 = tile_nz[tile + 1];
   const int nrows = (int)(x1 - x0);
@@ -150,20 +152,20 @@ mp_spmv_kernel(const Off* __restrict__ row_end, const int32_t* __restrict__ col,
     if (vec && q < end && nnz - origin >= q + E) {
       load_items<E>(cp, c);
       load_items<E>(vp, v);
-#pragma unroll
-      for (int j = 0; j < E; ++j) {
-        const bool in = q + j >= lead && q + j < end;
-        xv[j] = in ? __ldg(x + c[j]) : V(0);
-        if (!in) v[j] = V(0);
-      }
     } else {
 #pragma unroll
       for (int j = 0; j < E; ++j) {
         const bool in = q + j >= lead && q + j < end;
         c[j] = in ? ld_stream(cp + j) : 0;
         v[j] = in ? ld_stream(vp + j) : V(0);
-        xv[j] = in ? __ldg(x + c[j]) : V(0);
       }
+    }
+    wait_for_previous();
+#pragma unroll
+    for (int j = 0; j < E; ++j) {
+      const bool in = q + j >= lead && q + j < end;
+      xv[j] = in ? __ldg(x + c[j]) : V(0);
+      if (!in) v[j] = V(0);
     }
   }
 
@@ -265,6 +267,8 @@ __global__ void mp_fixup_kernel(const Off* __restrict__ carry_row, const V* __re
                                 long long num_tiles, Off n_rows, V* __restrict__ y) {
   constexpr unsigned kFull = 0xffffffffu;
   constexpr int kShort = 4;
+  release_next();
+  wait_for_previous();
   const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   const int lane = threadIdx.x & 31;
   Off r = n_rows;
@@ -311,7 +315,13 @@ bool launch_tiles(const MpMatrix& m, int threads, const void* x, void* y, cudaSt
     return false;
   }
   const bool vec = ((reinterpret_cast<uintptr_t>(m.col) | reinterpret_cast<uintptr_t>(m.val)) & 31) == 0;
-  kern<<<(unsigned)m.num_tiles, threads, (size_t)threads * (E * sizeof(unsigned short) + 2 * sizeof(V)), s>>>(
+  const size_t smem = (size_t)threads * (E * sizeof(unsigned short) + 2 * sizeof(V));
+  if (m.in_place)
+    return launch_chained(kern, (unsigned)m.num_tiles, threads, smem, s, static_cast<const Off*>(m.row_end), m.col,
+                          static_cast<const V*>(m.val), static_cast<const V*>(x), static_cast<V*>(y),
+                          static_cast<const Off*>(m.tile_row), static_cast<const Off*>(m.tile_nz), (Off)m.nnz, vec,
+                          static_cast<Off*>(m.carry_row), static_cast<V*>(m.carry_val));
+  kern<<<(unsigned)m.num_tiles, threads, smem, s>>>(
       static_cast<const Off*>(m.row_end), m.col, static_cast<const V*>(m.val), static_cast<const V*>(x),
       static_cast<V*>(y), static_cast<const Off*>(m.tile_row), static_cast<const Off*>(m.tile_nz), (Off)m.nnz, vec,
       static_cast<Off*>(m.carry_row), static_cast<V*>(m.carry_val));
@@ -337,10 +347,9 @@ bool launch_mp(const MpMatrix& m, const void* x, void* y, cudaStream_t s, cudaEv
   if (ev && !VNEC_CUDA(cudaEventRecord(ev[1], s))) return false;
   const int fb = 256;
   long long fg = (m.num_tiles + fb - 1) / fb;
-  mp_fixup_kernel<V, Off><<<(unsigned)fg, fb, 0, s>>>(static_cast<const Off*>(m.carry_row),
-                                                      static_cast<const V*>(m.carry_val), m.num_tiles,
-                                                      (Off)m.n_rows, static_cast<V*>(y));
-  if (!VNEC_CUDA(cudaGetLastError())) return false;
+  if (!launch_chained(mp_fixup_kernel<V, Off>, (unsigned)fg, fb, 0, s, static_cast<const Off*>(m.carry_row),
+                      static_cast<const V*>(m.carry_val), (long long)m.num_tiles, (Off)m.n_rows, static_cast<V*>(y)))
+    return false;
   if (ev && !VNEC_CUDA(cudaEventRecord(ev[2], s))) return false;
   return true;
 }

@@ -17,6 +17,7 @@
 #include <cstdint>
 
 #include "common.h"
+#include "launch.cuh"
 #include "long_rows.cuh"
 #include "prefetch.cuh"
 #include "sliced.h"
@@ -147,12 +148,16 @@ dense_block_kernel(const SlicedTask* __restrict__ tasks, long long num_tasks, co
                    int n_cols, V* __restrict__ y, V* __restrict__ chunk_sum) {
   const long long w = ((long long)blockIdx.x * kWarpsPerBlock) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
+  release_next();
   if (w >= num_tasks) return;
   const int4 raw = __ldg(reinterpret_cast<const int4*>(tasks) + w);
   const int base = raw.x, row_base = raw.y, steps = raw.z, meta = raw.w;
   const int kind = meta & 15, vwl = (meta >> 4) & 15, nrows = (meta >> 8) & 0xff;
+  const int g = lane >> vwl;
+  const int row = kind != kSlicedChunk && g < nrows ? __ldg(rowid + row_base + g) : 0;
+  wait_for_previous();
   if (kind == kSlicedZero) {
-    if (lane < nrows) y[rowid[row_base + lane]] = V(0);
+    if (lane < nrows) y[row] = V(0);
     return;
   }
   const V* vp = val + (size_t)(base + lane) * 4;
@@ -170,9 +175,8 @@ dense_block_kernel(const SlicedTask* __restrict__ tasks, long long num_tasks, co
   for (int off = (1 << vwl) >> 1; off > 0; off >>= 1) acc += __shfl_xor_sync(kFull, acc, off);
   if (kind == kSlicedChunk) {
     if (lane == 0) chunk_sum[row_base] = acc;
-  } else {
-    const int g = lane >> vwl;
-    if ((lane & ((1 << vwl) - 1)) == 0 && g < nrows) y[rowid[row_base + g]] = acc;
+  } else if ((lane & ((1 << vwl) - 1)) == 0 && g < nrows) {
+    y[row] = acc;
   }
 }
 
@@ -222,6 +226,7 @@ __device__ __forceinline__ void sliced_task(long long w, int lane, const SlicedT
         prefetch_l2_range(col + e0, len, lane);
     }
   }
+  wait_for_previous();
   if (kind == kSlicedZero) {
     if (lane < nrows) {
       const int row = rowid[row_base + lane];
@@ -306,6 +311,7 @@ sliced_kernel(const SlicedTask* __restrict__ tasks, long long num_tasks, const V
               SlicedEpilogue ep = SlicedEpilogue(), const uint16_t* __restrict__ col16 = nullptr,
               const int32_t* __restrict__ first = nullptr, SlicedPrefetch pf = SlicedPrefetch()) {
   const long long w = ((long long)blockIdx.x * kWarpsPerBlock) + (threadIdx.x >> 5);
+  release_next();
   if (w >= num_tasks) return;
   sliced_task<V, U, H, HOT, EPI>(w, threadIdx.x & 31, tasks, val, col, rowid, x, y, chunk_sum, xh, ncols, ep, col16,
                                  first, pf);
@@ -321,6 +327,8 @@ sliced_guard_kernel(const int* __restrict__ guard, const SlicedTask* __restrict_
                     const int32_t* __restrict__ rowid, const double* __restrict__ x, double* y,
                     double* __restrict__ chunk_sum, const double* __restrict__ xh, int ncols,
                     const uint16_t* __restrict__ col16, const int32_t* __restrict__ first) {
+  release_next();
+  wait_for_previous();
   if (*reinterpret_cast<const volatile int*>(guard) == 0) return;
   const SlicedEpilogue ep;
   const long long stride = (long long)gridDim.x * kWarpsPerBlock;
@@ -334,6 +342,8 @@ __global__ void sliced_long_fixup(const int32_t* __restrict__ long_row, const in
                                   const int32_t* __restrict__ long_heavy, long long num_long, long long num_heavy,
                                   long long heavy_sub, unsigned light_blocks, const V* __restrict__ chunk_sum, V* y,
                                   SlicedEpilogue ep = SlicedEpilogue()) {
+  release_next();
+  wait_for_previous();
   long_rows_fixup<V>(long_first, long_heavy, num_long, num_heavy, heavy_sub, light_blocks, chunk_sum,
                      [&](long long i, V s) {
                        const int row = long_row[i];
@@ -343,6 +353,8 @@ __global__ void sliced_long_fixup(const int32_t* __restrict__ long_row, const in
 
 template <typename V>
 __global__ void epilogue_kernel(V* y, long long n, SlicedEpilogue ep) {
+  release_next();
+  wait_for_previous();
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
     const double g = ep.gamma_dev ? fma(ep.gamma_dev_scale, *ep.gamma_dev, ep.gamma) : ep.gamma;
     double r = fma(ep.alpha, static_cast<double>(y[i]), g);
@@ -358,16 +370,24 @@ bool launch_dense(const SlicedMatrix& m, const void* x, void* y, cudaStream_t s)
     set_error("dense blocks: too many tasks for one launch");
     return false;
   }
-  dense_block_kernel<V><<<(unsigned)grid, kWarpsPerBlock * 32, 0, s>>>(
-      m.tasks, m.num_tasks, static_cast<const V*>(m.val), m.col, m.rowid, static_cast<const V*>(x), (int)m.n_cols,
-      static_cast<V*>(y), static_cast<V*>(m.chunk_sum));
-  return VNEC_CUDA(cudaGetLastError());
+  return launch_chained(dense_block_kernel<V>, (unsigned)grid, kWarpsPerBlock * 32, 0, s, m.tasks, m.num_tasks,
+                        static_cast<const V*>(m.val), m.col, m.rowid, static_cast<const V*>(x), (int)m.n_cols,
+                        static_cast<V*>(y), static_cast<V*>(m.chunk_sum));
 }
 
 template <typename V>
 __global__ void gather_hot(const V* __restrict__ x, const int32_t* __restrict__ hot_cols, int n, V* __restrict__ xh) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) xh[i] = __ldg(x + __ldg(hot_cols + i));
+  release_next();
+  const int c = i < n ? __ldg(hot_cols + i) : 0;
+  wait_for_previous();
+  if (i < n) xh[i] = __ldg(x + c);
+}
+
+template <typename V>
+bool launch_gather_hot(const SlicedMatrix& m, const void* x, cudaStream_t s) {
+  return launch_chained(gather_hot<V>, (unsigned)((m.hot + 255) / 256), 256, 0, s, static_cast<const V*>(x),
+                        m.hot_cols, m.hot, static_cast<V*>(m.xhot));
 }
 
 template <typename V, int U, int H, bool HOT, bool EPI = false>
@@ -385,17 +405,11 @@ bool launch_main(const SlicedMatrix& m, const void* x, void* y, cudaStream_t s,
     set_error("sliced: too many tasks for one launch");
     return false;
   }
-  if (HOT && !m.hot_ready) {
-    gather_hot<V><<<(unsigned)((m.hot + 255) / 256), 256, 0, s>>>(static_cast<const V*>(x), m.hot_cols, m.hot,
-                                                                  static_cast<V*>(m.xhot));
-    if (!VNEC_CUDA(cudaGetLastError())) return false;
-  }
-  kern<<<(unsigned)grid, kWarpsPerBlock * 32, 0, s>>>(m.tasks, m.num_tasks, static_cast<const V*>(m.val), m.col,
-                                                      m.rowid, static_cast<const V*>(x), static_cast<V*>(y),
-                                                      static_cast<V*>(m.chunk_sum),
-                                                      static_cast<const V*>(m.xhot), (int)m.n_cols, ep, m.col16,
-                                                      m.first, m.pf);
-  return VNEC_CUDA(cudaGetLastError());
+  if (HOT && !m.hot_ready && !launch_gather_hot<V>(m, x, s)) return false;
+  return launch_chained(kern, (unsigned)grid, kWarpsPerBlock * 32, 0, s, m.tasks, m.num_tasks,
+                        static_cast<const V*>(m.val), m.col, m.rowid, static_cast<const V*>(x), static_cast<V*>(y),
+                        static_cast<V*>(m.chunk_sum), static_cast<const V*>(m.xhot), (int)m.n_cols, ep, m.col16,
+                        m.first, m.pf);
 }
 
 template <typename V, int U, bool HOT>
@@ -454,15 +468,11 @@ bool launch(const SlicedMatrix& m, const void* x, void* y, cudaStream_t s, cudaE
   if (m.num_long > 0) {
     const int b = 128;
     const FixupGrid g = fixup_grid(m, b);
-    if (fused)
-      sliced_long_fixup<V, true><<<g.total, b, 0, s>>>(m.long_row, m.long_first, m.long_heavy, m.num_long,
-                                                       m.num_heavy, m.heavy_sub, g.light,
-                                                       static_cast<const V*>(m.chunk_sum), static_cast<V*>(y), *epi);
-    else
-      sliced_long_fixup<V><<<g.total, b, 0, s>>>(m.long_row, m.long_first, m.long_heavy, m.num_long, m.num_heavy,
-                                                 m.heavy_sub, g.light, static_cast<const V*>(m.chunk_sum),
-                                                 static_cast<V*>(y));
-    if (!VNEC_CUDA(cudaGetLastError())) return false;
+    auto kern = fused ? sliced_long_fixup<V, true> : sliced_long_fixup<V, false>;
+    if (!launch_chained(kern, g.total, b, 0, s, m.long_row, m.long_first, m.long_heavy, (long long)m.num_long,
+                        (long long)m.num_heavy, (long long)m.heavy_sub, g.light, static_cast<const V*>(m.chunk_sum),
+                        static_cast<V*>(y), fused ? *epi : SlicedEpilogue()))
+      return false;
   }
   if (epi && !fused && !apply_epilogue(y, m.n_rows, sizeof(V) == 8, *epi, s)) return false;
   if (ev && !VNEC_CUDA(cudaEventRecord(ev[2], s))) return false;
@@ -480,18 +490,14 @@ bool sliced_guard_f64(const SlicedMatrix& m, const double* x, double* y, const i
   const long long need = (m.num_tasks + kWarpsPerBlock - 1) / kWarpsPerBlock;
   const unsigned grid = (unsigned)std::max<long long>(1, std::min<long long>(need, 8LL * sms));
   if (m.hot > 0) {
-    gather_hot<double><<<(unsigned)((m.hot + 255) / 256), 256, 0, s>>>(x, m.hot_cols, m.hot,
-                                                                       static_cast<double*>(m.xhot));
-    if (!VNEC_CUDA(cudaGetLastError())) return false;
-    sliced_guard_kernel<true><<<grid, kWarpsPerBlock * 32, 0, s>>>(
-        flag, m.tasks, m.num_tasks, static_cast<const double*>(m.val), m.col, m.rowid, x, y,
-        static_cast<double*>(m.chunk_sum), static_cast<const double*>(m.xhot), (int)m.n_cols, m.col16, m.first);
-  } else {
-    sliced_guard_kernel<false><<<grid, kWarpsPerBlock * 32, 0, s>>>(
-        flag, m.tasks, m.num_tasks, static_cast<const double*>(m.val), m.col, m.rowid, x, y,
-        static_cast<double*>(m.chunk_sum), nullptr, 0, m.col16, m.first);
+    if (!launch_gather_hot<double>(m, x, s)) return false;
+    return launch_chained(sliced_guard_kernel<true>, grid, kWarpsPerBlock * 32, 0, s, flag, m.tasks, m.num_tasks,
+                          static_cast<const double*>(m.val), m.col, m.rowid, x, y, static_cast<double*>(m.chunk_sum),
+                          static_cast<const double*>(m.xhot), (int)m.n_cols, m.col16, m.first);
   }
-  return VNEC_CUDA(cudaGetLastError());
+  return launch_chained(sliced_guard_kernel<false>, grid, kWarpsPerBlock * 32, 0, s, flag, m.tasks, m.num_tasks,
+                        static_cast<const double*>(m.val), m.col, m.rowid, x, y, static_cast<double*>(m.chunk_sum),
+                        nullptr, 0, m.col16, m.first);
 }
 
 bool sliced_spmv(const SlicedMatrix& m, bool fp64, const void* x, void* y, cudaStream_t s, cudaEvent_t* ev,
@@ -501,23 +507,15 @@ bool sliced_spmv(const SlicedMatrix& m, bool fp64, const void* x, void* y, cudaS
 
 bool sliced_gather_hot(const SlicedMatrix& m, bool fp64, const void* x, cudaStream_t s) {
   if (m.hot <= 0) return true;
-  const unsigned g = (unsigned)((m.hot + 255) / 256);
-  if (fp64)
-    gather_hot<double><<<g, 256, 0, s>>>(static_cast<const double*>(x), m.hot_cols, m.hot, static_cast<double*>(m.xhot));
-  else
-    gather_hot<float><<<g, 256, 0, s>>>(static_cast<const float*>(x), m.hot_cols, m.hot, static_cast<float*>(m.xhot));
-  return VNEC_CUDA(cudaGetLastError());
+  return fp64 ? launch_gather_hot<double>(m, x, s) : launch_gather_hot<float>(m, x, s);
 }
 
 bool apply_epilogue(void* y, long long n, bool fp64, const SlicedEpilogue& e, cudaStream_t s) {
   if (n <= 0) return true;
   const int tb = 256;
   const unsigned grid = (unsigned)std::min<long long>((n + tb - 1) / tb, 152LL * 16);
-  if (fp64)
-    epilogue_kernel<double><<<grid, tb, 0, s>>>(static_cast<double*>(y), n, e);
-  else
-    epilogue_kernel<float><<<grid, tb, 0, s>>>(static_cast<float*>(y), n, e);
-  return VNEC_CUDA(cudaGetLastError());
+  return fp64 ? launch_chained(epilogue_kernel<double>, grid, tb, 0, s, static_cast<double*>(y), n, e)
+              : launch_chained(epilogue_kernel<float>, grid, tb, 0, s, static_cast<float*>(y), n, e);
 }
 
 }  // namespace vnec

@@ -28,6 +28,7 @@
 
 #include "common.h"
 #include "df32.cuh"
+#include "launch.cuh"
 #include "long_rows.cuh"
 #include "prefetch.cuh"
 #include "sliced.h"
@@ -119,6 +120,8 @@ __device__ __forceinline__ bool aligned16(const void* p) { return (reinterpret_c
 __device__ __forceinline__ void round_x(const double* __restrict__ x, float* __restrict__ x32, long long n,
                                         const int32_t* __restrict__ hot, int nh) {
   const long long t0 = blockIdx.x * (long long)blockDim.x + threadIdx.x, nt = (long long)gridDim.x * blockDim.x;
+  release_next();
+  wait_for_previous();
   const long long n4 = aligned16(x) && aligned16(x32) ? n / 4 : 0;
   for (long long q = t0; q < n4; q += nt) {
     const double2 a = __ldcs(reinterpret_cast<const double2*>(x) + 2 * q);
@@ -147,6 +150,8 @@ __global__ void x_to_f32_ext_kernel(const double* __restrict__ x, float* __restr
 __global__ void x_split_kernel(const double* __restrict__ x, float2* __restrict__ xs, long long n, int* flag,
                                const int32_t* __restrict__ hot, int nh) {
   const long long t0 = blockIdx.x * (long long)blockDim.x + threadIdx.x, nt = (long long)gridDim.x * blockDim.x;
+  release_next();
+  wait_for_previous();
   const long long n2 = aligned16(x) && aligned16(xs) ? n / 2 : 0;
   bool bad = false;
   for (long long q = t0; q < n2; q += nt) {
@@ -250,9 +255,9 @@ sliced_mixed_kernel(const SlicedTask* __restrict__ tasks, long long num_tasks, c
                     const signed char* __restrict__ chunk_scale, const int* __restrict__ flag,
                     const uint16_t* __restrict__ col16, const int32_t* __restrict__ first,
                     const uint16_t* __restrict__ pat16, SlicedPrefetch pf) {
-  if (flag && *reinterpret_cast<const volatile int*>(flag)) return;  // DF32: x out of range, guard launch computes
   const long long w = ((long long)blockIdx.x * kWarps) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
+  release_next();
   if (w >= num_tasks) return;
   const int4 raw = __ldg(reinterpret_cast<const int4*>(tasks) + w);
   const int base = raw.x, row_base = raw.y, steps = raw.z, meta = raw.w;
@@ -267,6 +272,8 @@ sliced_mixed_kernel(const SlicedTask* __restrict__ tasks, long long num_tasks, c
       if ((meta & kSlicedDelta) && !(SH && (meta & kSlicedShared))) prefetch_l2_range(col16 + e0, len, lane);
     }
   }
+  wait_for_previous();
+  if (flag && *reinterpret_cast<const volatile int*>(flag)) return;  // DF32: x out of range, guard launch computes
   if (kind == kSlicedZero) {
     if (lane < nrows) y[rowid[row_base + lane]] = 0.0;
     return;
@@ -566,12 +573,18 @@ __global__ void long_fixup_f64(const int32_t* __restrict__ long_row, const int32
                                const int32_t* __restrict__ long_heavy, long long num_long, long long num_heavy,
                                long long heavy_sub, unsigned light_blocks, const double* __restrict__ chunk_sum,
                                double* __restrict__ y, int* flag) {
+  release_next();
+  wait_for_previous();
   if (blockIdx.x == 0 && threadIdx.x == 0 && flag) *flag = 0;  // consumed: reset for the next call
   long_rows_fixup<double>(long_first, long_heavy, num_long, num_heavy, heavy_sub, light_blocks, chunk_sum,
                           [&](long long i, double s) { y[long_row[i]] = s; });
 }
 
-__global__ void reset_flag(int* flag) { *flag = 0; }
+__global__ void reset_flag(int* flag) {
+  release_next();
+  wait_for_previous();
+  *flag = 0;
+}
 
 template <class C>
 bool launch_mixed(const SlicedMatrix& m, const SlicedMixed& mx, const void* xs, double* y, cudaStream_t s,
@@ -603,10 +616,10 @@ bool launch_mixed(const SlicedMatrix& m, const SlicedMixed& mx, const void* xs, 
   auto kern = (R > 0 && m.lane_run) ? pick(std::integral_constant<int, R>{}) : pick(std::integral_constant<int, 0>{});
   // DF32 reads the pre-split (hi, lo) pairs; the FP64 values stay for the guard launch.
   const void* vals = std::is_same<typename C::Val, float2>::value ? static_cast<const void*>(mx.val_split) : m.val;
-  kern<<<(unsigned)grid, kWarps * 32, 0, s>>>(m.tasks, m.num_tasks, static_cast<const typename C::Val*>(vals), m.col,
-                                              m.rowid, xs, y, static_cast<double*>(m.chunk_sum), mx.row_scale,
-                                              mx.chunk_scale, flag, m.col16, m.first, m.pat16, m.pf);
-  return VNEC_CUDA(cudaGetLastError());
+  return launch_chained(kern, (unsigned)grid, kWarps * 32, 0, s, m.tasks, (long long)m.num_tasks,
+                        static_cast<const typename C::Val*>(vals), m.col, m.rowid, xs, y,
+                        static_cast<double*>(m.chunk_sum), mx.row_scale, mx.chunk_scale, flag, m.col16, m.first,
+                        m.pat16, m.pf);
 }
 
 }  // namespace
@@ -620,12 +633,14 @@ bool sliced_mixed_spmv(const SlicedMatrix& m, const SlicedMixed& mx, const doubl
   int* flag = nullptr;
   if (nx > 0) {
     if (mx.precision == kPrecDF32) {
-      x_split_kernel<<<xg, tb, 0, s>>>(x, static_cast<float2*>(mx.xbuf), nx, mx.flag, m.hot_cols, m.hot);
       flag = mx.flag;
-    } else {
-      x_to_f32_ext_kernel<<<xg, tb, 0, s>>>(x, static_cast<float*>(mx.xbuf), nx, m.hot_cols, m.hot);
+      if (!launch_chained(x_split_kernel, (unsigned)xg, tb, 0, s, x, static_cast<float2*>(mx.xbuf), nx, mx.flag,
+                          m.hot_cols, m.hot))
+        return false;
+    } else if (!launch_chained(x_to_f32_ext_kernel, (unsigned)xg, tb, 0, s, x, static_cast<float*>(mx.xbuf), nx,
+                               m.hot_cols, m.hot)) {
+      return false;
     }
-    if (!VNEC_CUDA(cudaGetLastError())) return false;
   }
   if (m.num_tasks > 0) {
     bool ok = false;
@@ -645,13 +660,12 @@ bool sliced_mixed_spmv(const SlicedMatrix& m, const SlicedMixed& mx, const doubl
   if (m.num_long > 0) {
     const int b = 128;
     const FixupGrid g = fixup_grid(m, b);
-    long_fixup_f64<<<g.total, b, 0, s>>>(m.long_row, m.long_first, m.long_heavy, m.num_long, m.num_heavy,
-                                         m.heavy_sub, g.light, static_cast<const double*>(m.chunk_sum), y,
-                                         mx.precision == kPrecDF32 ? mx.flag : nullptr);
-    if (!VNEC_CUDA(cudaGetLastError())) return false;
-  } else if (mx.precision == kPrecDF32) {
-    reset_flag<<<1, 1, 0, s>>>(mx.flag);
-    if (!VNEC_CUDA(cudaGetLastError())) return false;
+    if (!launch_chained(long_fixup_f64, g.total, b, 0, s, m.long_row, m.long_first, m.long_heavy,
+                        (long long)m.num_long, (long long)m.num_heavy, (long long)m.heavy_sub, g.light,
+                        static_cast<const double*>(m.chunk_sum), y, mx.precision == kPrecDF32 ? mx.flag : nullptr))
+      return false;
+  } else if (mx.precision == kPrecDF32 && !launch_chained(reset_flag, 1, 1, 0, s, mx.flag)) {
+    return false;
   }
   if (ev && !VNEC_CUDA(cudaEventRecord(ev[2], s))) return false;
   return true;
@@ -661,16 +675,14 @@ bool split_to_df32(const double* x, float2* xs, long long n, int* flag, cudaStre
   if (n <= 0) return true;
   const int tb = 256;
   const int grid = (int)std::min<long long>((n + tb - 1) / tb, 152LL * 16);
-  x_split_kernel<<<grid, tb, 0, s>>>(x, xs, n, flag, nullptr, 0);
-  return VNEC_CUDA(cudaGetLastError());
+  return launch_chained(x_split_kernel, (unsigned)grid, tb, 0, s, x, xs, n, flag, nullptr, 0);
 }
 
 bool round_to_f32(const double* x, float* x32, long long n, cudaStream_t s) {
   if (n <= 0) return true;
   const int tb = 256;
   const int grid = (int)std::min<long long>((n + tb - 1) / tb, 152LL * 16);
-  x_to_f32_kernel<<<grid, tb, 0, s>>>(x, x32, n);
-  return VNEC_CUDA(cudaGetLastError());
+  return launch_chained(x_to_f32_kernel, (unsigned)grid, tb, 0, s, x, x32, n);
 }
 
 }  // namespace vnec
@@ -684,6 +696,8 @@ extern "C" SpB_Info SpB_VNEC_f64_to_f32_ext(const double* d_in, float* d_out, in
   if (n == 0) return SpB_SUCCESS;
   const int tb = 256;
   const int grid = (int)std::min<long long>((n + tb - 1) / tb, 152LL * 16);
-  vnec::x_to_f32_kernel<<<grid, tb, 0, static_cast<cudaStream_t>(stream)>>>(d_in, d_out, n);
-  return VNEC_CUDA(cudaGetLastError()) ? SpB_SUCCESS : SpB_FAILURE;
+  return vnec::launch_chained(vnec::x_to_f32_kernel, (unsigned)grid, tb, 0, static_cast<cudaStream_t>(stream), d_in,
+                              d_out, (long long)n)
+             ? SpB_SUCCESS
+             : SpB_FAILURE;
 }

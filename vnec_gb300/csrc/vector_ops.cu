@@ -9,6 +9,7 @@
 #include <cstdint>
 
 #include "common.h"
+#include "launch.cuh"
 #include "vnec_gb300.h"
 
 namespace vnec {
@@ -30,6 +31,8 @@ __global__ void __launch_bounds__(kDotTpb)
 dot_partial_kernel(long long n, const double* __restrict__ a, const double* __restrict__ b, int mode,
                    double* __restrict__ partial) {
   __shared__ double sh[kDotTpb / 32];
+  release_next();
+  wait_for_previous();
   double acc = 0.0;
   for (long long i = (long long)blockIdx.x * kDotTpb + threadIdx.x; i < n; i += (long long)gridDim.x * kDotTpb)
     acc = mode == 0 ? fma(a[i], b[i], acc) : acc + fabs(a[i] - b[i]);
@@ -40,6 +43,8 @@ dot_partial_kernel(long long n, const double* __restrict__ a, const double* __re
 __global__ void __launch_bounds__(kDotTpb)
 dot_final_kernel(const double* __restrict__ partial, int n, double* __restrict__ out) {
   __shared__ double sh[kDotTpb / 32];
+  release_next();
+  wait_for_previous();
   double acc = 0.0;
   for (int i = threadIdx.x; i < n; i += kDotTpb) acc += partial[i];
   const double s = block_sum(acc, sh);
@@ -58,8 +63,9 @@ extern "C" SpB_Info SpB_VNEC_dot_ext(int64_t n, const double* d_a, const double*
     return SpB_FAILURE;
   }
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  dot_partial_kernel<<<SPB_VNEC_DOT_BLOCKS, kDotTpb, 0, s>>>(n, d_a, d_b, mode, d_partial);
-  if (!VNEC_CUDA(cudaGetLastError())) return SpB_FAILURE;
-  dot_final_kernel<<<1, kDotTpb, 0, s>>>(d_partial, SPB_VNEC_DOT_BLOCKS, d_out);
-  return VNEC_CUDA(cudaGetLastError()) ? SpB_SUCCESS : SpB_FAILURE;
+  return launch_chained(dot_partial_kernel, SPB_VNEC_DOT_BLOCKS, kDotTpb, 0, s, (long long)n, d_a, d_b, mode,
+                        d_partial) &&
+                 launch_chained(dot_final_kernel, 1, kDotTpb, 0, s, d_partial, SPB_VNEC_DOT_BLOCKS, d_out)
+             ? SpB_SUCCESS
+             : SpB_FAILURE;
 }
