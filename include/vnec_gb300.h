@@ -457,14 +457,18 @@ typedef struct {
                           SpB_VNEC_PREC_DF32 (values and X as FP32 hi+lo pairs, double-float products
                           and sums on the FP32 pipe: FP64-level error; needs |a| in [2^-40, 2^41) or 0,
                           a call whose X leaves that range computes in FP64) */
-  int lanes;           /* lanes per row (divides 32 and k, k / lanes in {1,2,4,8}); 0: tuned or default */
-  int long_row_len;    /* rows longer than this are cut into chunks; 0: tuned or 1024 */
+  int lanes;           /* lanes per row (divides 32 and k, k / lanes in {1,2,4,8}); 0: tuned, or k / 4
+                          (1 below k = 4; FP32: k for k <= 4).  With k / lanes >= 2 device x and y must be
+                          16-byte aligned, except with lanes 0 and k <= 4 */
+  int long_row_len;    /* rows longer than this are cut into chunks; 0: tuned, or 1024 for
+                          FP32, 256 below 2^22 nonzeros and for k >= 16, else 512 */
   int chunk;           /* entries per chunk; 0: long_row_len */
-  int warps_per_block; /* 4 or 8; 0: tuned or 8 */
+  int warps_per_block; /* 4 or 8; 0: tuned or 4 */
   int autotune;        /* 1: time candidate layouts on a sample of the batch and keep the fastest */
   int no_graph;        /* 1: launch the kernels directly on each call */
   int window_rows;     /* rows sorted by length within windows of this size (0: 65536) */
-  int max_steps;       /* a row group spreads over enough slots to take at most this many steps (0: 32) */
+  int max_steps;       /* a row group spreads over enough slots to take at most this many steps (0: 32,
+                          FP64 and DF32 16 for k <= 8 below 2^22 nonzeros) */
   int unroll;          /* kernel mode: 1 normal load steps in flight per lane, 2 doubled, 3 each
                           task's columns and values read in bulk (128 per round) and passed to
                           the slots by shuffles; 0: tuned or normal */

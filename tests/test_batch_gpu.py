@@ -405,3 +405,53 @@ def test_batch_k1_layout_option_checked(built, batch):
     for bad in (1, -2):
         with pytest.raises(api.VnecError, match="k1_layout"):
             api.BatchPlan(batch, 1, k1_layout=bad)
+
+
+@pytest.mark.parametrize("precision", [0, 1, 3], ids=["fp64", "fp32", "df32"])
+@pytest.mark.parametrize("k", [2, 4])
+def test_batch_default_layout_takes_any_alignment(built, batch, k, precision):
+    """The default layouts of k = 2 and 4 keep 2 or 4 right-hand sides in a lane
+    and still take device pointers that are only 8-byte aligned, with the bits
+    of the aligned call (for DF32 also on its FP64 guard path)."""
+    import torch
+
+    from vnec_gb300 import api
+
+    p = api.BatchPlan(batch, k, precision=precision)
+    ro, co = p.offsets()
+    for big in (False, True):
+        xv = _x(p, k)
+        if big:
+            xv[5] = 1e30  # outside the double-float range
+        want = p.mxv_host(xv).reshape(-1)
+        x = torch.zeros(int(co[-1]) * k + 1, dtype=torch.float64, device="cuda")
+        y = torch.zeros(int(ro[-1]) * k + 1, dtype=torch.float64, device="cuda")
+        x[1:] = torch.from_numpy(xv).cuda()
+        p.mxv_device(x.data_ptr() + 8, y.data_ptr() + 8, 0)
+        torch.cuda.synchronize()
+        assert y[1:].cpu().numpy().tobytes() == want.tobytes()
+        p.mxv_device(x.data_ptr() + 8, y.data_ptr(), 0)
+        torch.cuda.synchronize()
+        assert y[:-1].cpu().numpy().tobytes() == want.tobytes()
+    p.free()
+
+
+@pytest.mark.parametrize("k", [2, 8])
+def test_batch_fp32_widening(built, k):
+    """FP32 sums reach FP64 exactly: one product a row, over normal, subnormal,
+    zero, infinite and NaN results."""
+    from vnec_gb300 import api
+
+    a = np.array([1.0, -3.0, 2.0 ** -100, -2.0 ** -120, 2.0 ** 100, -2.0 ** 127, 0.0, 7.5])
+    xs = np.array([1.0, -2.0 ** -30, 2.0 ** -45, 2.0 ** 40, np.inf, np.nan, -0.0, 1.0 + 2.0 ** -23])
+    n = a.size
+    rp, col = np.arange(n * n + 1), np.tile(np.arange(n), n)
+    m = Csr(n * n, n, rp, col, np.repeat(a, n))
+    p = api.BatchPlan([m], k, precision=api.PREC_FP32)
+    X = np.repeat(xs[:, None], k, axis=1)
+    Y = p.mxv_host(X.reshape(-1)).reshape(n * n, k)
+    p.free()
+    with np.errstate(all="ignore"):
+        want = (np.repeat(a, n).astype(np.float32) * np.tile(xs, n).astype(np.float32)).astype(np.float64)
+    for r in range(k):
+        assert np.array_equal(Y[:, r], want, equal_nan=True)

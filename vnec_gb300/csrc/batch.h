@@ -37,6 +37,10 @@ struct BatchMatrix {
   int grid = 0;                         // persistent CTAs
   bool per_task = false;                // one warp per task (blocks dispatched in task order) instead of persistent warps
   int warps_per_block = 8;
+  // FP32: 2^n consecutive tasks per warp, with 2^n times k / lanes right-hand
+  // sides per lane; 0 (k / lanes <= 8), 1 (k / lanes = 4, or lanes = k = 2) or 2
+  // (lanes = k = 4), mode 0.
+  int tasks_log2 = 0;
   int mode = 0;                         // 0: U steps in flight, 1: 2U, 2: entries staged in registers
   int precision = 0;                    // kPrecFP64, kPrecFP32 or kPrecDF32 (SlicedPrecision)
   void* xbuf = nullptr;                 // FP32 / DF32: n_cols * k converted X

@@ -265,6 +265,9 @@ BatchHost* batch_build(int n, const int64_t* n_rows, const int64_t* n_cols, cons
         }
       }
     }
+    // Longest tasks first (chunks, then long rows): a chunk is several times a
+    // short row's work and would run alone at the end of the launch.
+    std::reverse(h->tasks.begin() + off_t[w], h->tasks.begin() + off_t[w + 1]);
   }
   h->long_first[(size_t)h->num_long] = (int32_t)h->num_chunks;
   return h;

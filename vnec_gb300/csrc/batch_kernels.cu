@@ -24,6 +24,20 @@
 //          (FP64-level accuracy), FP64 slot/chunk sums.  When the split kernel
 //          flags an X value outside the split range, the same launch computes
 //          in FP64 (value = hi + lo, FP64 X).
+//
+// What bounds it: FP64 from k = 8 on the FP64 pipe (17 M nonzeros, k = 32: 870 us
+// of FMAs in a 952 us call), the others the latency and requests of the X gathers.
+// So FP64 additions and conversions are kept few (slots are summed by halving the
+// right-hand sides a lane holds, FP32 sums are widened by integer operations), and
+// the FP32 and double-float loops fetch the next steps' columns and values before
+// they wait for X (FP64 loops do not: the registers cost more warps than it hides;
+// k = 32 971 -> 997 us).  Measured on lognormal batches of 17 M and, in brackets,
+// 0.8 M nonzeros, us a call, against one task per warp, slots summed by a full
+// butterfly, no fetch-ahead and half or a quarter of the right-hand sides per lane:
+//   k =        2               8               32
+//   FP64   187 -> 103      304 -> 264      1063 -> 952   (122 -> 43)
+//   FP32   129 -> 74       142 -> 111       410 -> 301   (60 -> 41)
+//   DF32   168 -> 92       218 -> 174       643 -> 586   (94 -> 30)
 
 #include <cuda_runtime.h>
 
@@ -60,10 +74,24 @@ struct BatchArgs {
   int llog2;  // lanes per slot L = 1 << llog2
 };
 
-// R consecutive elements of type T at p (16-, 8- or 4-byte vector loads).
-template <typename T, int R> __device__ __forceinline__ void load_vec(const T* p, T (&v)[R]) {
+// R consecutive elements of type T at p: 32-byte loads (WIDE, p aligned to 32
+// bytes: the library's own converted X) or 16-, 8- or 4-byte ones (VEC, p
+// aligned to the smaller of 16 bytes and the elements' size), else one by one.
+template <bool WIDE, bool VEC, typename T, int R> __device__ __forceinline__ void load_vec(const T* p, T (&v)[R]) {
   constexpr int bytes = R * (int)sizeof(T);
-  if constexpr (bytes >= 16) {
+  if constexpr (!VEC) {
+#pragma unroll
+    for (int r = 0; r < R; ++r) v[r] = __ldg(p + r);
+  } else if constexpr (WIDE && bytes >= 32) {
+#pragma unroll
+    for (int i = 0; i < bytes / 32; ++i) {
+      uint32_t w[8];
+      asm("ld.global.nc.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+          : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]), "=r"(w[4]), "=r"(w[5]), "=r"(w[6]), "=r"(w[7])
+          : "l"(reinterpret_cast<const char*>(p) + 32 * i));
+      memcpy(reinterpret_cast<char*>(v) + 32 * i, w, 32);
+    }
+  } else if constexpr (bytes >= 16) {
 #pragma unroll
     for (int i = 0; i < bytes / 16; ++i) {
       const int4 q = __ldg(reinterpret_cast<const int4*>(p) + i);
@@ -78,17 +106,32 @@ template <typename T, int R> __device__ __forceinline__ void load_vec(const T* p
   }
 }
 
-template <int R> __device__ __forceinline__ void store_y(double* p, const double (&v)[R]) {
-  if constexpr (R == 1) {
-    p[0] = v[0];
+// The first `n` of R values (n a power of two, uniform) to p.
+template <bool VEC, int R> __device__ __forceinline__ void store_y(double* p, const double (&v)[R], int n) {
+  if constexpr (VEC && R > 1) {
+#pragma unroll
+    for (int i = 0; i < R / 2; ++i)
+      if (2 * i + 1 < n) reinterpret_cast<double2*>(p)[i] = make_double2(v[2 * i], v[2 * i + 1]);
+    if (n == 1) p[0] = v[0];
   } else {
 #pragma unroll
-    for (int i = 0; i < R / 2; ++i) reinterpret_cast<double2*>(p)[i] = make_double2(v[2 * i], v[2 * i + 1]);
+    for (int i = 0; i < R; ++i)
+      if (i < n) p[i] = v[i];
   }
 }
 
+// An FP32 value as FP64 from its bits: normal numbers and zeros by integer
+// operations (a conversion takes the FP64 pipe of a warp for 16 cycles), the
+// rest by the instruction.
+__device__ __forceinline__ double widen(float f) {
+  const uint32_t b = __float_as_uint(f), e = (b >> 23) & 0xffu;
+  if (e - 1u < 254u)
+    return __hiloint2double((int)((b & 0x80000000u) | (((b & 0x7fffffffu) >> 3) + (896u << 20))), (int)(b << 29));
+  return (b << 1) == 0 ? __hiloint2double((int)b, 0) : static_cast<double>(f);
+}
+
 struct CodecF64 {
-  static constexpr bool kPairReduce = false;
+  static constexpr bool kPairReduce = false, kOwnX = false, kAhead = false;
   using V = double;
   using X = double;
   struct A {
@@ -100,7 +143,7 @@ struct CodecF64 {
 };
 
 struct CodecF32 {
-  static constexpr bool kPairReduce = false;
+  static constexpr bool kPairReduce = false, kOwnX = true, kAhead = true;
   using V = float;
   using X = float;
   struct A {
@@ -108,13 +151,13 @@ struct CodecF32 {
   };
   __device__ static A zero() { return A{0.f}; }
   __device__ static void mac(A& a, V v, X x) { a.s = fmaf(v, x, a.s); }
-  __device__ static double out(const A& a) { return static_cast<double>(a.s); }
+  __device__ static double out(const A& a) { return widen(a.s); }
 };
 
 // Double-float: value (hi, lo) times x (hi, lo), Dekker product with FMA,
 // TwoSum into (s, c).
 struct CodecDF32 {
-  static constexpr bool kPairReduce = true;
+  static constexpr bool kPairReduce = true, kOwnX = true, kAhead = true;
   using V = float2;
   using X = float2;
   struct A {
@@ -122,7 +165,17 @@ struct CodecDF32 {
   };
   // a += the (s, c) pair of the lane `off` away (TwoSum of the high parts).
   __device__ static void add_shfl(A& a, int off) {
-    const float s2 = __shfl_xor_sync(0xffffffffu, a.s, off), c2 = __shfl_xor_sync(0xffffffffu, a.c, off);
+    add(a, __shfl_xor_sync(0xffffffffu, a.s, off), __shfl_xor_sync(0xffffffffu, a.c, off));
+  }
+  // The lane keeps one of a and b (b in the upper lanes), gets that of the
+  // other lane and leaves the sum in a.
+  __device__ static void fold(A& a, const A& b, bool hi, int off) {
+    const A give = hi ? a : b, own = hi ? b : a;
+    const A got{__shfl_xor_sync(0xffffffffu, give.s, off), __shfl_xor_sync(0xffffffffu, give.c, off)};
+    a = hi ? got : own;  // the lower lane's pair first, whichever lane adds
+    add(a, hi ? own.s : got.s, hi ? own.c : got.c);
+  }
+  __device__ static void add(A& a, float s2, float c2) {
     const float t = __fadd_rn(a.s, s2);
     const float bb = __fsub_rn(t, a.s);
     const float e = __fadd_rn(__fsub_rn(a.s, __fsub_rn(t, bb)), __fsub_rn(s2, bb));
@@ -135,12 +188,12 @@ struct CodecDF32 {
     a.s = r.s;
     a.c = r.c;
   }
-  __device__ static double out(const A& a) { return df_to_f64(DF{a.s, a.c}); }
+  __device__ static double out(const A& a) { return widen(a.s) + widen(a.c); }
 };
 
 // FP64 from split values and FP64 X: the guard path of DF32 plans.
 struct CodecDF32Guard {
-  static constexpr bool kPairReduce = false;
+  static constexpr bool kPairReduce = false, kOwnX = false, kAhead = false;
   using V = float2;
   using X = double;
   struct A {
@@ -166,25 +219,36 @@ __device__ __forceinline__ float2 shfl_val(float2 v, int src) {
 // lanes (broadcast), U steps in flight.
 constexpr int kStageRounds = 4;
 
-template <class Cd, int R, int U, bool STAGED = false>
+//
+// TL > 0: a warp takes 2^TL consecutive tasks at once, W = 32 >> TL lanes each.
+// A layout of L lanes per slot then runs with L >> TL lanes that hold 2^TL times
+// the right-hand sides: every slot's sums are those of TL = 0, bit for bit, but
+// fewer lanes read each column and value and X comes in wider loads.
+template <class Cd, int R, int U, bool STAGED, bool VEC, int TL = 0>
 __device__ __forceinline__ void run_tasks(const BatchArgs& a, const typename Cd::X* __restrict__ x) {
+  static_assert(TL == 0 || (!STAGED && Cd::kAhead), "several tasks per warp run the fetch-ahead loop");
   using V = typename Cd::V;
   using X = typename Cd::X;
-  const int lane = threadIdx.x & 31;
+  constexpr int W = 32 >> TL;  // lanes of a task
+  const int lane = threadIdx.x & (W - 1);
   const int k = 1 << a.klog2;
-  const int S = 32 >> a.llog2;  // slots per step
-  const int slot = lane >> a.llog2, sub = lane & ((1 << a.llog2) - 1);
+  const int S = 32 >> a.llog2;      // slots per step
+  const int ll = a.llog2 - TL;      // lanes of a slot
+  const int slot = lane >> ll, sub = lane & ((1 << ll) - 1);
   const long long nw = (long long)gridDim.x * (blockDim.x >> 5);
   const V* __restrict__ val = static_cast<const V*>(a.val);
   const X* __restrict__ xs = x + sub * R;
-  for (long long t = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); t < a.num_tasks; t += nw) {
-    const int4 raw = __ldg(a.tasks + t);
-    const int base = raw.x, row_base = raw.y, steps = raw.z, kind = raw.w & 15, vwl = (raw.w >> 4) & 15,
-              nrows = raw.w >> 8;
+  for (long long w0 = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); w0 << TL < a.num_tasks;
+       w0 += nw) {
+    const long long t = (w0 << TL) + ((threadIdx.x & 31) >> (5 - TL));
+    // A warp's last tasks may be missing: no rows, no steps.
+    const int4 raw = TL == 0 || t < a.num_tasks ? __ldg(a.tasks + t) : make_int4(0, 0, 0, kSlicedZero);
+    const int base = raw.x, row_base = raw.y, kind = raw.w & 15, vwl = (raw.w >> 4) & 15, nrows = raw.w >> 8;
+    const int steps = TL > 0 && kind == kSlicedZero ? 0 : raw.z;
     if (kind == kSlicedZero) {
-      for (int i = lane; i < (nrows << a.klog2); i += 32)
+      for (int i = lane; i < (nrows << a.klog2); i += W)
         a.y[((size_t)__ldg(a.rowid + row_base + (i >> a.klog2)) << a.klog2) + (i & (k - 1))] = 0.0;
-      continue;
+      if (TL == 0) continue;
     }
     const V* vp = val + base + slot;
     const int32_t* cp = a.col + base + slot;
@@ -222,7 +286,7 @@ __device__ __forceinline__ void run_tasks(const BatchArgs& a, const typename Cd:
             X xv[U][R];
 #pragma unroll
             for (int u = 0; u < U; ++u)
-              if (j + u < spr && sb + j + u < steps) load_vec<X, R>(xs + ((size_t)c[u] << a.klog2), xv[u]);
+              if (j + u < spr && sb + j + u < steps) load_vec<Cd::kOwnX, VEC>(xs + ((size_t)c[u] << a.klog2), xv[u]);
 #pragma unroll
             for (int u = 0; u < U; ++u)
               if (j + u < spr && sb + j + u < steps)
@@ -233,90 +297,171 @@ __device__ __forceinline__ void run_tasks(const BatchArgs& a, const typename Cd:
       }
       s = steps;
     }
-    for (; s + U <= steps; s += U) {
-      int c[U];
-      V v[U];
+    if constexpr (Cd::kAhead) {
+      // U steps at a time; the next U steps' columns and values are fetched before
+      // these steps' X rows are waited for.
+      if (s < steps) {
+        int c[U];
+        V v[U];
 #pragma unroll
-      for (int u = 0; u < U; ++u) {
-        c[u] = __ldcs(cp + (s + u) * S);
-        v[u] = __ldcs(vp + (s + u) * S);
+        for (int u = 0; u < U; ++u)
+          if (u < steps) {
+            c[u] = __ldcs(cp + u * S);
+            v[u] = __ldcs(vp + u * S);
+          }
+        for (; s < steps; s += U) {
+          X xv[U][R];
+          V w[U];
+#pragma unroll
+          for (int u = 0; u < U; ++u)
+            if (s + u < steps) {
+              load_vec<Cd::kOwnX, VEC>(xs + ((size_t)c[u] << a.klog2), xv[u]);
+              w[u] = v[u];
+            }
+#pragma unroll
+          for (int u = 0; u < U; ++u)
+            if (s + U + u < steps) {
+              c[u] = __ldcs(cp + (s + U + u) * S);
+              v[u] = __ldcs(vp + (s + U + u) * S);
+            }
+#pragma unroll
+          for (int u = 0; u < U; ++u)
+            if (s + u < steps)
+#pragma unroll
+              for (int r = 0; r < R; ++r) Cd::mac(acc[r], w[u], xv[u][r]);
+        }
       }
-      X xv[U][R];
+    } else {
+      for (; s + U <= steps; s += U) {
+        int c[U];
+        V v[U];
 #pragma unroll
-      for (int u = 0; u < U; ++u) load_vec<X, R>(xs + ((size_t)c[u] << a.klog2), xv[u]);
+        for (int u = 0; u < U; ++u) {
+          c[u] = __ldcs(cp + (s + u) * S);
+          v[u] = __ldcs(vp + (s + u) * S);
+        }
+        X xv[U][R];
 #pragma unroll
-      for (int u = 0; u < U; ++u)
+        for (int u = 0; u < U; ++u) load_vec<Cd::kOwnX, VEC>(xs + ((size_t)c[u] << a.klog2), xv[u]);
 #pragma unroll
-        for (int r = 0; r < R; ++r) Cd::mac(acc[r], v[u], xv[u][r]);
-    }
-    for (; s < steps; ++s) {
-      const int c = __ldcs(cp + s * S);
-      const V v = __ldcs(vp + s * S);
-      X xv[R];
-      load_vec<X, R>(xs + ((size_t)c << a.klog2), xv);
+        for (int u = 0; u < U; ++u)
 #pragma unroll
-      for (int r = 0; r < R; ++r) Cd::mac(acc[r], v, xv[r]);
+          for (int r = 0; r < R; ++r) Cd::mac(acc[r], v[u], xv[u][r]);
+      }
+      for (; s < steps; ++s) {
+        const int c = __ldcs(cp + s * S);
+        const V v = __ldcs(vp + s * S);
+        X xv[R];
+        load_vec<Cd::kOwnX, VEC>(xs + ((size_t)c << a.klog2), xv);
+#pragma unroll
+        for (int r = 0; r < R; ++r) Cd::mac(acc[r], v, xv[r]);
+      }
     }
     // Slots to sum: the whole warp for a chunk, the V slots of a row otherwise.
-    const int span = kind == kSlicedChunk ? 32 : 1 << (a.llog2 + vwl);
+    // At each level the two halves of the lanes split the right-hand sides they
+    // still hold, so R values over n slots take R - 1 or fewer additions per lane
+    // instead of R log2(n); every sum is the butterfly's.
+    const int span = kind == kSlicedZero ? 0 : kind == kSlicedChunk ? W : 1 << (ll + vwl);
     double d[R];
+    int width = R, at = 0;  // this lane ends with right-hand sides [at, at + width) of its R
+    bool writes = true;
     if constexpr (Cd::kPairReduce) {
       // Double-float: sum the slots as (hi, lo) pairs on the FP32 pipe and
       // convert once (each FP64 operation costs 64 FP32 issue slots here).
-      for (int off = 1 << a.llog2; off < span; off <<= 1)
 #pragma unroll
-        for (int r = 0; r < R; ++r) Cd::add_shfl(acc[r], off);
+      for (int lev = 0; lev < 5; ++lev) {
+        const int off = 1 << (ll + lev);
+        if (off >= span) break;
+        const bool hi = (lane & off) != 0;
+        if ((R >> lev) > 1) {
 #pragma unroll
-      for (int r = 0; r < R; ++r) d[r] = Cd::out(acc[r]);
+          for (int j = 0; j < (R >> lev) / 2; ++j) Cd::fold(acc[j], acc[j + (R >> lev) / 2], hi, off);
+          width >>= 1;
+          at += hi ? width : 0;
+        } else {
+          Cd::add_shfl(acc[0], off);
+          writes = writes && !hi;
+        }
+      }
+#pragma unroll
+      for (int r = 0; r < R; ++r)
+        if (r < width) d[r] = Cd::out(acc[r]);
     } else {
 #pragma unroll
       for (int r = 0; r < R; ++r) d[r] = Cd::out(acc[r]);
-      for (int off = 1 << a.llog2; off < span; off <<= 1)
 #pragma unroll
-        for (int r = 0; r < R; ++r) d[r] += __shfl_xor_sync(kFull, d[r], off);
+      for (int lev = 0; lev < 5; ++lev) {
+        const int off = 1 << (ll + lev);
+        const bool adds = off < span;  // the same for all lanes of a task
+        if (TL == 0 ? !adds : !__any_sync(kFull, adds)) break;
+        const bool hi = (lane & off) != 0;
+        if ((R >> lev) > 1) {
+#pragma unroll
+          for (int j = 0; j < (R >> lev) / 2; ++j) {
+            const double keep = hi ? d[j + (R >> lev) / 2] : d[j], give = hi ? d[j] : d[j + (R >> lev) / 2];
+            const double sum = keep + __shfl_xor_sync(kFull, give, off);
+            if (adds) d[j] = sum;
+          }
+          if (adds) {
+            width >>= 1;
+            at += hi ? width : 0;
+          }
+        } else {
+          const double sum = d[0] + __shfl_xor_sync(kFull, d[0], off);
+          if (adds) {
+            d[0] = sum;
+            writes = writes && !hi;
+          }
+        }
+      }
     }
-    if (kind == kSlicedChunk) {
-      if (slot == 0) store_y<R>(a.chunk_sum + ((size_t)row_base << a.klog2) + sub * R, d);
+    if (TL == 0 ? kind == kSlicedChunk : __any_sync(kFull, kind == kSlicedChunk)) {
+      const bool chunk = kind == kSlicedChunk;
+      if (chunk && writes) store_y<VEC>(a.chunk_sum + ((size_t)row_base << a.klog2) + sub * R + at, d, width);
       __threadfence();
       __syncwarp();
-      const int li = __ldg(a.chunk_long + row_base);
-      const int c0 = __ldg(a.long_first + li), c1 = __ldg(a.long_first + li + 1);
-      int last = 0;
-      if (lane == 0) last = atomicAdd(a.chunk_count + li, 1) == c1 - c0 - 1;
-      last = __shfl_sync(kFull, last, 0);
+      int li = 0, c0 = 0, c1 = 0, last = 0;
+      if (chunk) {
+        li = __ldg(a.chunk_long + row_base);
+        c0 = __ldg(a.long_first + li);
+        c1 = __ldg(a.long_first + li + 1);
+        if (lane == 0) last = atomicAdd(a.chunk_count + li, 1) == c1 - c0 - 1;
+      }
+      last = __shfl_sync(kFull, last, 0, W);
       if (last) {
         __threadfence();
         const size_t yrow = (size_t)__ldg(a.long_row + li) << a.klog2;
-        for (int j = lane; j < k; j += 32) {
+        for (int j = lane; j < k; j += W) {
           double sum = 0.0;
           for (int c = c0; c < c1; ++c) sum += __ldcg(a.chunk_sum + ((size_t)c << a.klog2) + j);
           a.y[yrow + j] = sum;
         }
         if (lane == 0) a.chunk_count[li] = 0;
       }
-    } else {
+    }
+    if (kind == kSlicedRows) {
       const int g = slot >> vwl;
-      if ((slot & ((1 << vwl) - 1)) == 0 && g < nrows)
-        store_y<R>(a.y + ((size_t)__ldg(a.rowid + row_base + g) << a.klog2) + sub * R, d);
+      if (writes && g < nrows)
+        store_y<VEC>(a.y + ((size_t)__ldg(a.rowid + row_base + g) << a.klog2) + sub * R + at, d, width);
     }
   }
 }
 
-template <class Cd, int R, int U, bool STAGED>
+template <class Cd, int R, int U, bool STAGED, bool VEC, int TL = 0>
 __global__ void __launch_bounds__(256) batch_kernel(const BatchArgs a) {
   release_next();
   wait_for_previous();
-  run_tasks<Cd, R, U, STAGED>(a, static_cast<const typename Cd::X*>(a.x));
+  run_tasks<Cd, R, U, STAGED, VEC, TL>(a, static_cast<const typename Cd::X*>(a.x));
 }
 
-template <int R, int U, bool STAGED>
+template <int R, int U, bool STAGED, bool VEC>
 __global__ void __launch_bounds__(256) batch_df32_kernel(const BatchArgs a) {
   release_next();
   wait_for_previous();
   if (*reinterpret_cast<const volatile int*>(a.flag))
-    run_tasks<CodecDF32Guard, R, U, STAGED>(a, a.x64);
+    run_tasks<CodecDF32Guard, R, U, STAGED, VEC>(a, a.x64);
   else
-    run_tasks<CodecDF32, R, U, STAGED>(a, static_cast<const float2*>(a.x));
+    run_tasks<CodecDF32, R, U, STAGED, VEC>(a, static_cast<const float2*>(a.x));
 }
 
 // Steps in flight per lane: 8 / R (at least 2), doubled in mode 1; mode 2
@@ -324,26 +469,43 @@ __global__ void __launch_bounds__(256) batch_df32_kernel(const BatchArgs a) {
 template <int R, int MODE> constexpr int unroll_for() { return (R >= 4 ? 2 : 8 / R) * (MODE == 1 ? 2 : 1); }
 
 using BatchKernel = void (*)(BatchArgs);
-template <int R, int MODE> BatchKernel kernel_for(int precision) {
+template <int R, int MODE, bool VEC> BatchKernel kernel_for(int precision) {
   constexpr int U = unroll_for<R, MODE>();
   constexpr bool ST = MODE == 2;
   switch (precision) {
-    case kPrecFP32: return &batch_kernel<CodecF32, R, U, ST>;
-    case kPrecDF32: return &batch_df32_kernel<R, U, ST>;
-    default: return &batch_kernel<CodecF64, R, U, ST>;
+    case kPrecFP32: return &batch_kernel<CodecF32, R, U, ST, VEC>;
+    case kPrecDF32: return &batch_df32_kernel<R, U, ST, VEC>;
+    default: return &batch_kernel<CodecF64, R, U, ST, VEC>;
   }
 }
 
-template <int R> BatchKernel kernel_for_mode(int precision, int mode) {
-  return mode == 2 ? kernel_for<R, 2>(precision) : mode == 1 ? kernel_for<R, 1>(precision) : kernel_for<R, 0>(precision);
+template <int R, bool VEC = true> BatchKernel kernel_for_mode(int precision, int mode) {
+  return mode == 2   ? kernel_for<R, 2, VEC>(precision)
+         : mode == 1 ? kernel_for<R, 1, VEC>(precision)
+                     : kernel_for<R, 0, VEC>(precision);
 }
 
-BatchKernel pick_kernel(int precision, int r, int mode) {
+// Several FP32 tasks per warp (BatchMatrix::tasks_log2), by the right-hand sides
+// per lane: 8 with two tasks, 4 with four (k = 4), 2 with two (k = 2).
+BatchKernel pick_shared(int r, int tasks_log2, bool vec) {
+  if (r == 8 && tasks_log2 == 1) return &batch_kernel<CodecF32, 8, unroll_for<8, 0>(), false, true, 1>;
+  if (r == 4 && tasks_log2 == 2)
+    return vec ? &batch_kernel<CodecF32, 4, unroll_for<4, 0>(), false, true, 2>
+               : &batch_kernel<CodecF32, 4, unroll_for<4, 0>(), false, false, 2>;
+  if (r == 2 && tasks_log2 == 1)
+    return vec ? &batch_kernel<CodecF32, 2, unroll_for<2, 0>(), false, true, 1>
+               : &batch_kernel<CodecF32, 2, unroll_for<2, 0>(), false, false, 1>;
+  return nullptr;
+}
+
+// `vec`: X and Y are 16-byte aligned.  Layouts of 2 and 4 right-hand sides per
+// lane also run without (plans whose layout the caller did not fix).
+BatchKernel pick_kernel(int precision, int r, int mode, bool vec = true) {
   switch (r) {
     case 1: return kernel_for_mode<1>(precision, mode);
-    case 2: return kernel_for_mode<2>(precision, mode);
-    case 4: return kernel_for_mode<4>(precision, mode);
-    case 8: return kernel_for_mode<8>(precision, mode);
+    case 2: return vec ? kernel_for_mode<2>(precision, mode) : kernel_for_mode<2, false>(precision, mode);
+    case 4: return vec ? kernel_for_mode<4>(precision, mode) : kernel_for_mode<4, false>(precision, mode);
+    case 8: return vec ? kernel_for_mode<8>(precision, mode) : nullptr;
     default: return nullptr;
   }
 }
@@ -377,7 +539,7 @@ bool batch_spmm_range(const BatchMatrix& m, const double* X, double* Y, cudaStre
     set_error("batch: unsupported k / lanes");
     return false;
   }
-  const int R = m.k / m.lanes;
+  const int R = (m.k / m.lanes) << m.tasks_log2;
   const void* xin = X;
   const long long off = (long long)c0 * m.k, nx = (long long)(c1 - c0) * m.k;
   if (m.precision == kPrecFP32) {
@@ -406,11 +568,18 @@ bool batch_spmm_range(const BatchMatrix& m, const double* X, double* Y, cudaStre
   a.y = Y;
   a.klog2 = log2i(m.k);
   a.llog2 = log2i(m.lanes);
-  const BatchKernel fn = pick_kernel(m.precision, R, m.mode);
+  const bool vec = ((reinterpret_cast<uintptr_t>(X) | reinterpret_cast<uintptr_t>(Y)) & 15) == 0;
+  const BatchKernel fn =
+      m.tasks_log2 > 0 ? pick_shared(R, m.tasks_log2, vec) : pick_kernel(m.precision, R, m.mode, vec || R == 1);
+  if (!fn) {
+    set_error("batch: x and y must be 16-byte aligned for this plan's layout");
+    return false;
+  }
   // Persistent warps stride the task list; with per_task every warp takes one
   // task and the hardware dispatches the blocks in task order, so the tasks in
   // flight stay a compact window of the list (and of X's rows).
-  const long long per_task_grid = (a.num_tasks + m.warps_per_block - 1) / m.warps_per_block;
+  const long long per_block = (long long)m.warps_per_block << m.tasks_log2;
+  const long long per_task_grid = (a.num_tasks + per_block - 1) / per_block;
   if (m.per_task && per_task_grid > 0x7fffffffLL) {
     set_error("batch: too many tasks for one launch with one warp per task");
     return false;

@@ -164,7 +164,7 @@ BatchHost* build_host(const BatchSource& s, const std::vector<int>& pick, int k,
 // ---------------------------------------------------------------------------
 
 struct TuneChoice {
-  int lanes = 0, long_len = 1024, wpb = 8;
+  int lanes = 0, long_len = 512, wpb = 4;
   int deep = 0;  // kernel mode: 1 twice the load steps in flight, 2 entries staged in registers
   // One warp per task (blocks dispatched in task order) instead of persistent
   // warps striding the task list.  The default: on the 512-matrix batch it
@@ -418,6 +418,9 @@ struct BatchPlan final : Plan {
   TuneRun tuning;
   int precision = kPrecFP64;
   bool use_graph = true;
+  // x and y need not be 16-byte aligned: layouts the caller did not fix, of at
+  // most 4 right-hand sides (one lane's 2 or 4 then load and store one by one).
+  bool any_alignment = false;
   std::vector<int64_t> row_off, col_off;
   // Graph of the last (x, y) pair.
   std::mutex gmu;
@@ -551,7 +554,7 @@ struct BatchPlan final : Plan {
 
   bool run(const void* d_x, void* d_y, cudaStream_t s) override {
     const int R = k1 ? 1 : d.m.k / d.m.lanes;
-    if (R >= 2 && ((reinterpret_cast<uintptr_t>(d_x) | reinterpret_cast<uintptr_t>(d_y)) & 15)) {
+    if (R >= 2 && !any_alignment && ((reinterpret_cast<uintptr_t>(d_x) | reinterpret_cast<uintptr_t>(d_y)) & 15)) {
       set_error("batch: x and y must be 16-byte aligned for this plan's layout");
       return false;
     }
@@ -631,6 +634,39 @@ void plan_parts(BatchPlan* p, const BatchHostView& hv, int n_parts) {
     c_done = c1;
     w0 = w1;
   }
+}
+
+// Default layout (measured on batches of 0.5 to 100 M nonzeros, lognormal rows,
+// every k and form).
+//
+// Right-hand sides per lane: FP64 and DF32 up to 4, as many as one lane loads in
+// 32 bytes, so the fewest lanes read each column and value (17 M nonzeros, FP64,
+// us at k = 2, 4, 8, 16, 32: 103, 146, 268, 496, 953 against 133, 182, 316, 598,
+// 1100 with half as many).  The FP32 form keeps one per lane up to k = 4, then 4:
+// the slots a row is spread over decide how its FP32 sums round.  It gets its wide
+// loads from several tasks per warp (default_tasks_log2).
+int default_lanes(int k, int precision) {
+  return precision == kPrecFP32 ? (k >= 8 ? k / 4 : k) : k / std::min(k, 4);
+}
+int default_tasks_log2(int k, int precision) {
+  return precision != kPrecFP32 || k == 1 ? 0 : k == 4 ? 2 : 1;
+}
+
+// Rows longer than this become chunks of it.  A chunk is one warp's work from
+// start to end, so where a batch is small, or its FP64 (or double-float) work per
+// entry large, long chunks run alone at the end: 0.5 M nonzeros, k = 32, FP64: 100
+// us at 1024, 45 at 256; 17 M: 1015 against 952.  Short ones cost partial sums
+// (17 M, k = 2, FP64: 103 at 512, 109 at 256).  FP32: 1024 always, as above.
+int default_long_len(int k, int precision, int64_t nnz) {
+  if (precision == kPrecFP32) return 1024;
+  return nnz < ((int64_t)1 << 22) || k >= 16 ? 256 : 512;
+}
+
+// Steps a row takes at most: a lane holds a whole row's right-hand sides at small
+// k, so a small batch fills the GPU only with rows split over more slots (0.8 M
+// nonzeros, k = 2, FP64: 18.6 us at 32 steps, 12.5 at 16; 3.5 M: 39 against 31).
+int default_steps(int k, int precision, int64_t nnz) {
+  return precision != kPrecFP32 && k <= 8 && nnz < ((int64_t)1 << 22) ? 16 : 32;
 }
 
 // A k = 1 batch as one sliced plan: the block-diagonal concatenation (matrix
@@ -761,9 +797,8 @@ std::unique_ptr<Plan> build_batch(int n, const CsrView* mats, int k, const SpB_V
   }
 
   TuneChoice choice;
-  choice.lanes = o.lanes > 0 ? o.lanes : std::min(k, 32);
-  if (o.lanes == 0 && k >= 8) choice.lanes = k / 4;  // four right-hand sides per lane
-  if (o.long_row_len > 0) choice.long_len = o.long_row_len;
+  choice.lanes = o.lanes > 0 ? o.lanes : default_lanes(k, o.precision);
+  choice.long_len = o.long_row_len > 0 ? o.long_row_len : default_long_len(k, o.precision, p->nnz);
   if (o.warps_per_block > 0) choice.wpb = o.warps_per_block;
   if (o.unroll > 0) choice.deep = o.unroll - 1;
   bool fresh = false;  // layout tuned here: the dispatch is then decided on the whole batch
@@ -793,7 +828,8 @@ std::unique_ptr<Plan> build_batch(int n, const CsrView* mats, int k, const SpB_V
   p->prm.long_len = choice.long_len;
   p->prm.chunk = o.chunk > 0 ? o.chunk : choice.long_len;
   if (o.window_rows > 0) p->prm.window_rows = o.window_rows;
-  if (o.max_steps > 0) p->prm.max_steps = o.max_steps;
+  p->prm.max_steps = o.max_steps > 0 ? o.max_steps : o.autotune ? p->prm.max_steps : default_steps(k, o.precision, p->nnz);
+  p->any_alignment = o.lanes == 0 && k <= 4;
   std::vector<int> all((size_t)n);
   for (int m = 0; m < n; ++m) all[(size_t)m] = m;
   BatchHost* h = build_host(src, all, k, p->prm);
@@ -817,6 +853,7 @@ std::unique_ptr<Plan> build_batch(int n, const CsrView* mats, int k, const SpB_V
     tune_cache()[key] = choice;
     cache_file_store(key, choice);
   }
+  if (o.lanes == 0 && !o.autotune && choice.deep == 0) p->d.m.tasks_log2 = default_tasks_log2(k, o.precision);
   p->d.m.per_task = o.dispatch == 0 ? choice.per_task : o.dispatch == 2;
   if (ok) plan_parts(p.get(), batch_view(h), o.host_parts > 0 ? o.host_parts : 8);
   batch_free(h);
