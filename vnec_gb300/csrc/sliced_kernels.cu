@@ -129,23 +129,23 @@ template <> struct Quad<float> {
   }
 };
 
-template <typename V>
-__device__ __forceinline__ V block_dot(const V* vp, int c, const V* __restrict__ x, int n_cols, V acc) {
-  V v[4];
-  Quad<V>::load(vp, v);
-#pragma unroll
-  for (int l = 0; l < 4; ++l) {
-    const V xv = (c + l < n_cols) ? __ldg(x + c + l) : V(0);
-    acc = fmav<V>(v[l], xv, acc);
-  }
-  return acc;
-}
+// One warp per task, kDenseAhead<V> blocks of a lane in flight: their columns and
+// values are loaded together (the values do not wait for the columns), then their
+// x, and the last round is predicated instead of taking its blocks one by one.
+// What bounds it: latency (a block's columns, then its x; DRAM 40% busy before),
+// and for FP64 the FP64 pipe on filled-up blocks.  FP32 blocks of 24 x 24, 500,003
+// rows: 18.6 -> 12.6 us (4, 5, 8 blocks ahead: 12.9, 13.9, 13.4); band of 65:
+// 12.6 -> 9.7; lognormal rows, mostly one nonzero a block: 71 -> 65 (6) but 74
+// with 4 or 8 (4 needs more registers there).  FP64 at 4: band of 65 23.2 -> 19.7,
+// stencil 100^3 67.7 -> 67.5 (2: 64.9, but 98 -> 104 on lognormal rows).
+template <typename V> constexpr int kDenseAhead = sizeof(V) == 8 ? 4 : 6;
 
 template <typename V>
 __global__ void __launch_bounds__(kWarpsPerBlock * 32)
 dense_block_kernel(const SlicedTask* __restrict__ tasks, long long num_tasks, const V* __restrict__ val,
                    const int32_t* __restrict__ col, const int32_t* __restrict__ rowid, const V* __restrict__ x,
                    int n_cols, V* __restrict__ y, V* __restrict__ chunk_sum) {
+  constexpr int U = kDenseAhead<V>;
   const long long w = ((long long)blockIdx.x * kWarpsPerBlock) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   release_next();
@@ -153,30 +153,39 @@ dense_block_kernel(const SlicedTask* __restrict__ tasks, long long num_tasks, co
   const int4 raw = __ldg(reinterpret_cast<const int4*>(tasks) + w);
   const int base = raw.x, row_base = raw.y, steps = raw.z, meta = raw.w;
   const int kind = meta & 15, vwl = (meta >> 4) & 15, nrows = (meta >> 8) & 0xff;
-  const int g = lane >> vwl;
-  const int row = kind != kSlicedChunk && g < nrows ? __ldg(rowid + row_base + g) : 0;
   wait_for_previous();
   if (kind == kSlicedZero) {
-    if (lane < nrows) y[row] = V(0);
+    if (lane < nrows) y[rowid[row_base + lane]] = V(0);
     return;
   }
   const V* vp = val + (size_t)(base + lane) * 4;
   const int32_t* cp = col + base + lane;
   V acc = V(0);
-  int k = 0;
-  for (; k + 4 <= steps; k += 4) {
-    int c[4];
+  for (int k = 0; k < steps; k += U) {
+    int c[U];
+    V v[U][4];
 #pragma unroll
-    for (int u = 0; u < 4; ++u) c[u] = __ldcs(cp + (k + u) * 32);
+    for (int u = 0; u < U; ++u)
+      if (k + u < steps) {
+        c[u] = __ldcs(cp + (k + u) * 32);
+        Quad<V>::load(vp + (size_t)(k + u) * 128, v[u]);
+      }
 #pragma unroll
-    for (int u = 0; u < 4; ++u) acc = block_dot<V>(vp + (size_t)(k + u) * 128, c[u], x, n_cols, acc);
+    for (int u = 0; u < U; ++u)
+      if (k + u < steps) {
+        V xv[4];
+#pragma unroll
+        for (int l = 0; l < 4; ++l) xv[l] = c[u] + l < n_cols ? __ldg(x + c[u] + l) : V(0);
+#pragma unroll
+        for (int l = 0; l < 4; ++l) acc = fmav<V>(v[u][l], xv[l], acc);
+      }
   }
-  for (; k < steps; ++k) acc = block_dot<V>(vp + (size_t)k * 128, __ldcs(cp + k * 32), x, n_cols, acc);
   for (int off = (1 << vwl) >> 1; off > 0; off >>= 1) acc += __shfl_xor_sync(kFull, acc, off);
   if (kind == kSlicedChunk) {
     if (lane == 0) chunk_sum[row_base] = acc;
-  } else if ((lane & ((1 << vwl) - 1)) == 0 && g < nrows) {
-    y[row] = acc;
+  } else {
+    const int g = lane >> vwl;
+    if ((lane & ((1 << vwl) - 1)) == 0 && g < nrows) y[rowid[row_base + g]] = acc;
   }
 }
 
