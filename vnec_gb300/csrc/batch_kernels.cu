@@ -120,16 +120,6 @@ template <bool VEC, int R> __device__ __forceinline__ void store_y(double* p, co
   }
 }
 
-// An FP32 value as FP64 from its bits: normal numbers and zeros by integer
-// operations (a conversion takes the FP64 pipe of a warp for 16 cycles), the
-// rest by the instruction.
-__device__ __forceinline__ double widen(float f) {
-  const uint32_t b = __float_as_uint(f), e = (b >> 23) & 0xffu;
-  if (e - 1u < 254u)
-    return __hiloint2double((int)((b & 0x80000000u) | (((b & 0x7fffffffu) >> 3) + (896u << 20))), (int)(b << 29));
-  return (b << 1) == 0 ? __hiloint2double((int)b, 0) : static_cast<double>(f);
-}
-
 struct CodecF64 {
   static constexpr bool kPairReduce = false, kOwnX = false, kAhead = false;
   using V = double;
@@ -188,7 +178,7 @@ struct CodecDF32 {
     a.s = r.s;
     a.c = r.c;
   }
-  __device__ static double out(const A& a) { return widen(a.s) + widen(a.c); }
+  __device__ static double out(const A& a) { return df_to_f64(DF{a.s, a.c}); }
 };
 
 // FP64 from split values and FP64 X: the guard path of DF32 plans.

@@ -1,9 +1,11 @@
-// Double-float arithmetic on the FP32 pipe (a value held as an unevaluated sum
-// hi + lo of two floats), shared by the DF32 forms of the merge-path, sliced
-// and batched kernels.  GB300 runs FP64 FMA at 1/64 of the FP32 rate; these
-// operations give products and sums with ~2^-46 relative error from FP32
-// instructions only.
+// Exact FP32 -> FP64 widening without the FP64 pipe, and double-float arithmetic
+// on the FP32 pipe (a value held as an unevaluated sum hi + lo of two floats),
+// shared by the precision forms of the merge-path, sliced and batched kernels.
+// GB300 runs FP64 FMA at 1/64 of the FP32 rate; these operations give products
+// and sums with ~2^-46 relative error from FP32 instructions only.
 #pragma once
+
+#include <cstdint>
 
 namespace vnec {
 
@@ -48,6 +50,16 @@ __device__ __forceinline__ DF df_mac(DF acc, float ah, float al, float xh, float
   return DF{t, __fadd_rn(acc.c, __fadd_rn(r, q))};
 }
 
-__device__ __forceinline__ double df_to_f64(DF a) { return static_cast<double>(a.s) + static_cast<double>(a.c); }
+// An FP32 value as FP64 from its bits: normal numbers and zeros by integer
+// operations (a conversion takes the FP64 pipe of a warp for 16 cycles), the
+// rest by the instruction.
+__device__ __forceinline__ double widen(float f) {
+  const uint32_t b = __float_as_uint(f), e = (b >> 23) & 0xffu;
+  if (e - 1u < 254u)
+    return __hiloint2double((int)((b & 0x80000000u) | (((b & 0x7fffffffu) >> 3) + (896u << 20))), (int)(b << 29));
+  return (b << 1) == 0 ? __hiloint2double((int)b, 0) : static_cast<double>(f);
+}
+
+__device__ __forceinline__ double df_to_f64(DF a) { return widen(a.s) + widen(a.c); }
 
 }  // namespace vnec

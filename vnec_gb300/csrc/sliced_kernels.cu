@@ -20,6 +20,7 @@
 #include "launch.cuh"
 #include "long_rows.cuh"
 #include "prefetch.cuh"
+#include "shared_pattern.cuh"
 #include "sliced.h"
 
 namespace vnec {
@@ -212,24 +213,28 @@ __device__ __forceinline__ V epi_out(V acc, int row, const SlicedEpilogue& ep) {
 }
 
 // One warp task (the body of sliced_kernel and of the DF32 guard kernel).
-template <typename V, int U, int H, bool HOT, bool EPI>
+// SH: the plan has shared-pattern tasks; plans without them run the SH = false
+// build, whose registers that path does not raise.
+template <typename V, int U, int H, bool HOT, bool EPI, bool SH = false>
 __device__ __forceinline__ void sliced_task(long long w, int lane, const SlicedTask* __restrict__ tasks,
                                             const V* __restrict__ val, const int32_t* __restrict__ col,
                                             const int32_t* __restrict__ rowid, const V* __restrict__ x, V* y,
                                             V* __restrict__ chunk_sum, const V* __restrict__ xh, int ncols,
                                             const SlicedEpilogue& ep, const uint16_t* __restrict__ col16,
                                             const int32_t* __restrict__ first,
-                                            const SlicedPrefetch& pf = SlicedPrefetch()) {
+                                            const SlicedPrefetch& pf = SlicedPrefetch(),
+                                            const uint16_t* __restrict__ pat16 = nullptr, int* s_off = nullptr) {
   const int4 raw = __ldg(reinterpret_cast<const int4*>(tasks) + w);
   const int base = raw.x, row_base = raw.y, steps = raw.z, meta = raw.w;
   const int kind = meta & 15, vwl = (meta >> 4) & 15, nrows = (meta >> 8) & 0xff;
   // The entries and task metadata ahead of this task, into L2 (prefetch.cuh).
   if (pf.entries > 0) {
-    prefetch_l2_task_meta(pf, w, base, row_base, kind != kSlicedChunk, tasks, first, rowid, nullptr, lane);
+    prefetch_l2_task_meta(pf, w, base, row_base, kind != kSlicedChunk, tasks, first, rowid, SH ? pat16 : nullptr, lane);
     const long long e0 = base + pf.entries, len = 32LL * steps;
     if (kind != kSlicedZero && e0 + len <= pf.n_entries) {
       prefetch_l2_range(val + e0, len, lane);
-      if (meta & kSlicedDelta)
+      if (SH && (meta & kSlicedShared)) {
+      } else if (meta & kSlicedDelta)
         prefetch_l2_range(col16 + e0, len, lane);
       else
         prefetch_l2_range(col + e0, len, lane);
@@ -240,6 +245,44 @@ __device__ __forceinline__ void sliced_task(long long w, int lane, const SlicedT
     if (lane < nrows) {
       const int row = rowid[row_base + lane];
       y[row] = epi_out<EPI>(V(0), row, ep);
+    }
+    return;
+  }
+  if (SH && (meta & kSlicedShared)) {
+    // One row per lane, all with the same column gaps (shared_pattern.cuh).
+    const int4* offs = pattern_offsets(pat16 + (base >> 5), steps, lane, s_off);
+    const V* xr = x + (lane < nrows ? __ldg(first + row_base + lane) : 0);
+    const V* vp = val + base + lane;
+    V acc = V(0);
+    int k = 0;
+    for (; k + U <= steps; k += U) {
+      V v[U], xv[U];
+      int o[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) v[u] = __ldcs(vp + (k + u) * 32);
+      pattern_at<U>(offs, k, o);
+#pragma unroll
+      for (int u = 0; u < U; ++u) xv[u] = __ldg(xr + o[u]);
+#pragma unroll
+      for (int u = 0; u < U; ++u) acc = fmav<V>(v[u], xv[u], acc);
+    }
+    for (; k < steps; k += 4) {
+      V v[4], xv[4];
+      int o[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (k + u < steps) v[u] = __ldcs(vp + (k + u) * 32);
+      pattern_at<4>(offs, k, o);
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (k + u < steps) xv[u] = __ldg(xr + o[u]);
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (k + u < steps) acc = fmav<V>(v[u], xv[u], acc);
+    }
+    if (lane < nrows) {
+      const int row = rowid[row_base + lane];
+      y[row] = epi_out<EPI>(acc, row, ep);
     }
     return;
   }
@@ -312,18 +355,20 @@ __device__ __forceinline__ void sliced_task(long long w, int lane, const SlicedT
   }
 }
 
-template <typename V, int U, int H, bool HOT = false, bool EPI = false>
+template <typename V, int U, int H, bool HOT = false, bool EPI = false, bool SH = false>
 __global__ void __launch_bounds__(kWarpsPerBlock * 32)
 sliced_kernel(const SlicedTask* __restrict__ tasks, long long num_tasks, const V* __restrict__ val,
               const int32_t* __restrict__ col, const int32_t* __restrict__ rowid, const V* __restrict__ x,
               V* y, V* __restrict__ chunk_sum, const V* __restrict__ xh = nullptr, int ncols = 0,
               SlicedEpilogue ep = SlicedEpilogue(), const uint16_t* __restrict__ col16 = nullptr,
-              const int32_t* __restrict__ first = nullptr, SlicedPrefetch pf = SlicedPrefetch()) {
+              const int32_t* __restrict__ first = nullptr, SlicedPrefetch pf = SlicedPrefetch(),
+              const uint16_t* __restrict__ pat16 = nullptr) {
+  __shared__ __align__(16) int s_off[SH ? kWarpsPerBlock : 1][kPatternSteps];
   const long long w = ((long long)blockIdx.x * kWarpsPerBlock) + (threadIdx.x >> 5);
   release_next();
   if (w >= num_tasks) return;
-  sliced_task<V, U, H, HOT, EPI>(w, threadIdx.x & 31, tasks, val, col, rowid, x, y, chunk_sum, xh, ncols, ep, col16,
-                                 first, pf);
+  sliced_task<V, U, H, HOT, EPI, SH>(w, threadIdx.x & 31, tasks, val, col, rowid, x, y, chunk_sum, xh, ncols, ep,
+                                     col16, first, pf, pat16, s_off[SH ? threadIdx.x >> 5 : 0]);
 }
 
 // FP64 recompute of a DF32 call whose x left the split range: a small grid of
@@ -399,14 +444,14 @@ bool launch_gather_hot(const SlicedMatrix& m, const void* x, cudaStream_t s) {
                         m.hot_cols, m.hot, static_cast<V*>(m.xhot));
 }
 
-template <typename V, int U, int H, bool HOT, bool EPI = false>
+template <typename V, int U, int H, bool HOT, bool EPI = false, bool SH = false>
 bool launch_main(const SlicedMatrix& m, const void* x, void* y, cudaStream_t s,
                  const SlicedEpilogue& ep = SlicedEpilogue()) {
-  auto kern = sliced_kernel<V, U, H, HOT, EPI>;
-  // No shared memory: give the whole unified L1/shared array to L1.
+  auto kern = sliced_kernel<V, U, H, HOT, EPI, SH>;
+  // No shared memory (SH: 1 KB a block): give the unified L1/shared array to L1.
   static std::atomic<unsigned long long> configured{0};  // per instantiation, per device
   if (!once_per_device(configured, [&] {
-        return VNEC_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 0));
+        return VNEC_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, SH ? 12 : 0));
       }))
     return false;
   const long long grid = (m.num_tasks + kWarpsPerBlock - 1) / kWarpsPerBlock;
@@ -418,11 +463,14 @@ bool launch_main(const SlicedMatrix& m, const void* x, void* y, cudaStream_t s,
   return launch_chained(kern, (unsigned)grid, kWarpsPerBlock * 32, 0, s, m.tasks, m.num_tasks,
                         static_cast<const V*>(m.val), m.col, m.rowid, static_cast<const V*>(x), static_cast<V*>(y),
                         static_cast<V*>(m.chunk_sum), static_cast<const V*>(m.xhot), (int)m.n_cols, ep, m.col16,
-                        m.first, m.pf);
+                        m.first, m.pf, m.pat16);
 }
 
 template <typename V, int U, bool HOT>
 bool launch_hints(const SlicedMatrix& m, const void* x, void* y, cudaStream_t s) {
+  // Shared-pattern tasks need 16-bit deltas, which a hot-column window rules out.
+  if constexpr (!HOT)
+    if (m.pat16 && m.cache_hints == 0) return launch_main<V, U, 0, false, false, true>(m, x, y, s);
   switch (m.cache_hints) {
     case 1: return launch_main<V, U, 1, HOT>(m, x, y, s);
     case 2: return launch_main<V, U, 2, HOT>(m, x, y, s);
@@ -443,6 +491,13 @@ bool launch_unroll(const SlicedMatrix& m, const void* x, void* y, cudaStream_t s
 
 template <typename V, bool HOT>
 bool launch_fused(const SlicedMatrix& m, const void* x, void* y, cudaStream_t s, const SlicedEpilogue& ep) {
+  if constexpr (!HOT)
+    if (m.pat16) switch (m.unroll) {
+        case 4: return launch_main<V, 4, 0, false, true, true>(m, x, y, s, ep);
+        case 8: return launch_main<V, 8, 0, false, true, true>(m, x, y, s, ep);
+        case 16: return launch_main<V, 16, 0, false, true, true>(m, x, y, s, ep);
+        default: return launch_main<V, 12, 0, false, true, true>(m, x, y, s, ep);
+      }
   switch (m.unroll) {
     case 4: return launch_main<V, 4, 0, HOT, true>(m, x, y, s, ep);
     case 8: return launch_main<V, 8, 0, HOT, true>(m, x, y, s, ep);

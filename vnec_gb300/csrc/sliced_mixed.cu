@@ -31,6 +31,7 @@
 #include "launch.cuh"
 #include "long_rows.cuh"
 #include "prefetch.cuh"
+#include "shared_pattern.cuh"
 #include "sliced.h"
 #include "vnec_gb300.h"
 
@@ -172,26 +173,29 @@ __global__ void x_split_kernel(const double* __restrict__ x, float2* __restrict_
 struct CodecF32 {
   using Val = float;
   using Acc = float;
+  __device__ static const void* at(const void* xs, int c) { return static_cast<const float*>(xs) + c; }
   __device__ static Acc zero() { return 0.0f; }
   __device__ static Acc mac(Acc a, Val v, const void* xs, int c) {
     return fmaf(v, __ldg(static_cast<const float*>(xs) + c), a);
   }
-  __device__ static double to_f64(Acc a) { return static_cast<double>(a); }
+  __device__ static double to_f64(Acc a) { return widen(a); }
 };
 
 struct CodecBF16 {
   using Val = unsigned short;
   using Acc = float;
+  __device__ static const void* at(const void* xs, int c) { return static_cast<const float*>(xs) + c; }
   __device__ static Acc zero() { return 0.0f; }
   __device__ static Acc mac(Acc a, Val v, const void* xs, int c) {
     return fmaf(__uint_as_float(static_cast<unsigned>(v) << 16), __ldg(static_cast<const float*>(xs) + c), a);
   }
-  __device__ static double to_f64(Acc a) { return static_cast<double>(a); }
+  __device__ static double to_f64(Acc a) { return widen(a); }
 };
 
 struct CodecDF32 {
   using Val = float2;  // (hi, lo) split at plan build (the range was checked there)
   using Acc = DF;
+  __device__ static const void* at(const void* xs, int c) { return static_cast<const float2*>(xs) + c; }
   __device__ static Acc zero() { return DF{0.0f, 0.0f}; }
   __device__ static Acc mac(Acc acc, Val v, const void* xs, int c) {
     const float2 x = __ldg(static_cast<const float2*>(xs) + c);
@@ -238,8 +242,11 @@ __device__ __forceinline__ T run_at(const uint32_t (&w)[N], int t) {
   }
 }
 
-__device__ __forceinline__ double pow2(int e) {
-  return __longlong_as_double(static_cast<long long>(e + 1023) << 52);
+// s * 2^e for |e| <= 120 and s zero, infinite, NaN or of magnitude 2^-149 to
+// 2^200 (sums of FP32 values): the exponent moved by an integer addition.
+__device__ __forceinline__ double scale2(double s, int e) {
+  const int hi = __double2hiint(s), x = (hi >> 20) & 0x7ff;
+  return x - 1u < 2046u ? __hiloint2double(hi + (e << 20), __double2loint(s)) : s;
 }
 
 // P > 0: the arrays hold lane runs of P steps (SlicedMatrix::lane_run);
@@ -289,22 +296,16 @@ sliced_mixed_kernel(const SlicedTask* __restrict__ tasks, long long num_tasks, c
   constexpr bool kSerialTail = sizeof(Val) == 2;
   constexpr int UBS = U / 4 > 0 ? U / 4 : 1;
   if (SH && (meta & kSlicedShared)) {
-    // Every row of the task has `steps` entries with the same column gaps:
-    // lane k loads gap k of the shared pattern, a warp prefix sum turns the
-    // gaps into offsets from the first column, and step k's column is the
-    // row's first column plus offset k (a shuffle; no load on the x path).
-    int off = lane < steps ? __ldg(pat16 + (base >> 5) + lane) : 0;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int t = __shfl_up_sync(0xffffffffu, off, o);
-      if (lane >= o) off += t;
-    }
-    const int c0 = lane < nrows ? __ldg(first + row_base + lane) : 0;
+    // Every row of the task has `steps` entries with the same column gaps
+    // (shared_pattern.cuh).
+    __shared__ __align__(16) int s_off[kWarps][kPatternSteps];
+    const int4* offs = pattern_offsets(pat16 + (base >> 5), steps, lane, s_off[threadIdx.x >> 5]);
+    const void* xr = C::at(xs, lane < nrows ? __ldg(first + row_base + lane) : 0);
     typename C::Acc acc = C::zero();
     const Val* vp = val + base + lane;
-    if constexpr (P > 0 && kSerialTail) {
-      // BF16 runs: UBS runs at a time, then single runs, then the tail one
-      // step at a time (fewer registers than a preloaded 7-step tail).
+    if constexpr (P > 0) {
+      // Lane runs of P steps: UBS runs at a time, then single runs, then the
+      // stride-32 tail.
       const int nb = steps / P;
       const Val* vr = val + base + lane * P;
       int b = 0;
@@ -313,60 +314,59 @@ sliced_mixed_kernel(const SlicedTask* __restrict__ tasks, long long num_tasks, c
 #pragma unroll
         for (int u = 0; u < UBS; ++u) ld_words(vr + (b + u) * 32 * P, vw[u]);
 #pragma unroll
-        for (int u = 0; u < UBS; ++u)
+        for (int u = 0; u < UBS; ++u) {
+          int o[P];
+          pattern_at<P>(offs, (b + u) * P, o);
 #pragma unroll
-          for (int t = 0; t < P; ++t)
-            acc = C::mac(acc, run_at<Val>(vw[u], t), xs, c0 + __shfl_sync(0xffffffffu, off, (b + u) * P + t));
+          for (int t = 0; t < P; ++t) acc = C::mac(acc, run_at<Val>(vw[u], t), xr, o[t]);
+        }
       }
       for (; b < nb; ++b) {
         uint32_t vw[VW];
+        int o[P];
         ld_words(vr + b * 32 * P, vw);
+        pattern_at<P>(offs, b * P, o);
 #pragma unroll
-        for (int t = 0; t < P; ++t)
-          acc = C::mac(acc, run_at<Val>(vw, t), xs, c0 + __shfl_sync(0xffffffffu, off, b * P + t));
+        for (int t = 0; t < P; ++t) acc = C::mac(acc, run_at<Val>(vw, t), xr, o[t]);
       }
-      for (int k = nb * P; k < steps; ++k)
-        acc = C::mac(acc, ld_stream(vp + k * 32), xs, c0 + __shfl_sync(0xffffffffu, off, k));
-    } else if constexpr (P > 0) {
-      // Lane runs of P steps, UB runs per round (the last round predicated),
-      // then the stride-32 tail, whose values load with the first round.
-      const int nb = steps / P, k0 = nb * P;
-      Val tv[TL];
+      for (int k = nb * P; k < steps; k += 4) {
+        Val v[4];
+        int o[4];
 #pragma unroll
-      for (int t = 0; t < TL; ++t)
-        if (k0 + t < steps) tv[t] = ld_stream(vp + (k0 + t) * 32);
-      const Val* vr = val + base + lane * P;
-      for (int b = 0; b < nb; b += UB) {
-        uint32_t vw[UB][VW];
-#pragma unroll
-        for (int u = 0; u < UB; ++u)
-          if (b + u < nb) ld_words(vr + (b + u) * 32 * P, vw[u]);
-#pragma unroll
-        for (int u = 0; u < UB; ++u)
-          if (b + u < nb) {
-#pragma unroll
-            for (int t = 0; t < P; ++t)
-              acc = C::mac(acc, run_at<Val>(vw[u], t), xs, c0 + __shfl_sync(0xffffffffu, off, (b + u) * P + t));
-          }
-      }
-#pragma unroll
-      for (int t = 0; t < TL; ++t)
-        if (k0 + t < steps) acc = C::mac(acc, tv[t], xs, c0 + __shfl_sync(0xffffffffu, off, k0 + t));
-    } else {
-      // Chunks of U steps, the last one predicated.
-      for (int k = 0; k < steps; k += U) {
-        Val v[U];
-#pragma unroll
-        for (int u = 0; u < U; ++u)
+        for (int u = 0; u < 4; ++u)
           if (k + u < steps) v[u] = ld_stream(vp + (k + u) * 32);
+        pattern_at<4>(offs, k, o);
 #pragma unroll
-        for (int u = 0; u < U; ++u)
-          if (k + u < steps) acc = C::mac(acc, v[u], xs, c0 + __shfl_sync(0xffffffffu, off, k + u));
+        for (int u = 0; u < 4; ++u)
+          if (k + u < steps) acc = C::mac(acc, v[u], xr, o[u]);
+      }
+    } else {
+      // U steps at a time, then groups of four, the last one predicated.
+      int k = 0;
+      for (; k + U <= steps; k += U) {
+        Val v[U];
+        int o[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) v[u] = ld_stream(vp + (k + u) * 32);
+        pattern_at<U>(offs, k, o);
+#pragma unroll
+        for (int u = 0; u < U; ++u) acc = C::mac(acc, v[u], xr, o[u]);
+      }
+      for (; k < steps; k += 4) {
+        Val v[4];
+        int o[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+          if (k + u < steps) v[u] = ld_stream(vp + (k + u) * 32);
+        pattern_at<4>(offs, k, o);
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+          if (k + u < steps) acc = C::mac(acc, v[u], xr, o[u]);
       }
     }
     if (lane < nrows) {
       const double s = C::to_f64(acc);
-      y[rowid[row_base + lane]] = row_scale ? s * pow2(row_scale[row_base + lane]) : s;
+      y[rowid[row_base + lane]] = row_scale ? scale2(s, row_scale[row_base + lane]) : s;
     }
     return;
   }
@@ -413,7 +413,7 @@ sliced_mixed_kernel(const SlicedTask* __restrict__ tasks, long long num_tasks, c
       }
       if (lane < nrows) {
         const double s = C::to_f64(acc);
-        y[rowid[row_base + lane]] = row_scale ? s * pow2(row_scale[row_base + lane]) : s;
+        y[rowid[row_base + lane]] = row_scale ? scale2(s, row_scale[row_base + lane]) : s;
       }
       return;
     } else if constexpr (P > 0) {
@@ -456,7 +456,7 @@ sliced_mixed_kernel(const SlicedTask* __restrict__ tasks, long long num_tasks, c
         }
       if (lane < nrows) {
         const double s = C::to_f64(acc);
-        y[row] = row_scale ? s * pow2(row_scale[row_base + lane]) : s;
+        y[row] = row_scale ? scale2(s, row_scale[row_base + lane]) : s;
       }
       return;
     }
@@ -481,7 +481,7 @@ sliced_mixed_kernel(const SlicedTask* __restrict__ tasks, long long num_tasks, c
     }
     if (lane < nrows) {
       const double s = C::to_f64(acc);
-      y[rowid[row_base + lane]] = row_scale ? s * pow2(row_scale[row_base + lane]) : s;
+      y[rowid[row_base + lane]] = row_scale ? scale2(s, row_scale[row_base + lane]) : s;
     }
     return;
   }
@@ -561,11 +561,11 @@ sliced_mixed_kernel(const SlicedTask* __restrict__ tasks, long long num_tasks, c
   double s = C::to_f64(acc);
   for (int off = (1 << vwl) >> 1; off > 0; off >>= 1) s += __shfl_xor_sync(kFull, s, off);
   if (kind == kSlicedChunk) {
-    if (lane == 0) chunk_sum[row_base] = chunk_scale ? s * pow2(chunk_scale[row_base]) : s;
+    if (lane == 0) chunk_sum[row_base] = chunk_scale ? scale2(s, chunk_scale[row_base]) : s;
   } else {
     const int g = lane >> vwl;
     if ((lane & ((1 << vwl) - 1)) == 0 && g < nrows)
-      y[rowid[row_base + g]] = row_scale ? s * pow2(row_scale[row_base + g]) : s;
+      y[rowid[row_base + g]] = row_scale ? scale2(s, row_scale[row_base + g]) : s;
   }
 }
 

@@ -646,9 +646,9 @@ std::unique_ptr<Plan> build_sliced(const CsrView& v, const SpB_VNEC_options_ext*
   // 16-bit column deltas where rows allow them (not with a hot window, whose
   // relabelled columns break the increasing order).
   p->prm.delta16 = p->prm.hot == 0 && !(opts && opts->column_deltas < 0);
-  // Shared-pattern tasks: read by the precision forms' kernel (the FP64
-  // kernel walks the per-lane deltas, which stay stored).
-  p->prm.shared = p->prm.delta16 && prec != kPrecFP64 && !(opts && opts->shared_patterns < 0);
+  // Shared-pattern tasks (the per-lane deltas stay stored: the DF32 form's FP64
+  // guard and the cache-hint variants walk them).
+  p->prm.shared = p->prm.delta16 && !(opts && opts->shared_patterns < 0);
   SlicedHost* h = sliced_build(v.n_rows, v.n_cols, v.ptr, v.ptr64, cols, cols64, src_val, vb, p->prm, 1, keep);
   if (!h) {
     set_error("sliced format: more than 2^31 entries or row slots");
