@@ -1,11 +1,19 @@
 // Device reductions for chains of SpMV calls that stay on the GPU (power
 // iterations: a dangling-mass dot product, an L1 convergence distance).  Two
-// launches with a fixed summation order, so the result has the same bits on
-// every run: SPB_VNEC_DOT_BLOCKS blocks write partial sums, one block adds
-// them in block order.
+// launches with a summation order fixed by n and the vectors' alignment, so the
+// result has the same bits on every run: up to SPB_VNEC_DOT_BLOCKS blocks write
+// partial sums, one block adds them in block order.
+//
+// Bound by latency at these sizes (2^20 values are 16.8 MB, 2.5 us at HBM rate):
+// a thread has eight values of each vector in flight as 16-byte loads, into four
+// sums, and a short vector takes fewer blocks.  One value at a time and always
+// 1,024 blocks before: 16,384 values 7.2 -> 4.8 us, 2^20 10.0 -> 8.9 (differences
+// 12.6 -> 11.4); long vectors run at HBM rate as before (5 10^7: 124 us, products;
+// differences 238 -> 210, two FP64 instructions a value).
 
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdint>
 
 #include "common.h"
@@ -27,16 +35,47 @@ __device__ __forceinline__ double block_sum(double v, double* sh) {
   return s;
 }
 
+constexpr int kDotPairs = 4;  // pairs of values in flight per thread
+constexpr long long kDotBlockValues = (long long)kDotTpb * 2 * kDotPairs;
+
+// MODE 0: products; 1: absolute differences (compiled apart: chosen at run time,
+// both were computed, three FP64 instructions a value).  `vec`: both vectors are
+// 16-byte aligned.
+template <int MODE>
 __global__ void __launch_bounds__(kDotTpb)
-dot_partial_kernel(long long n, const double* __restrict__ a, const double* __restrict__ b, int mode,
+dot_partial_kernel(long long n, const double* __restrict__ a, const double* __restrict__ b, bool vec,
                    double* __restrict__ partial) {
   __shared__ double sh[kDotTpb / 32];
   release_next();
   wait_for_previous();
-  double acc = 0.0;
-  for (long long i = (long long)blockIdx.x * kDotTpb + threadIdx.x; i < n; i += (long long)gridDim.x * kDotTpb)
-    acc = mode == 0 ? fma(a[i], b[i], acc) : acc + fabs(a[i] - b[i]);
-  const double s = block_sum(acc, sh);
+  auto add = [](double acc, double u, double v) {
+    if constexpr (MODE == 0)
+      return fma(u, v, acc);
+    else
+      return acc + fabs(u - v);
+  };
+  double acc[kDotPairs] = {};
+  const long long t = (long long)blockIdx.x * kDotTpb + threadIdx.x, stride = (long long)gridDim.x * kDotTpb;
+  const long long n2 = vec ? n / 2 : 0;
+  const double2 *a2 = reinterpret_cast<const double2*>(a), *b2 = reinterpret_cast<const double2*>(b);
+  long long q = t;
+  for (; q + (kDotPairs - 1) * stride < n2; q += kDotPairs * stride) {
+    double2 u[kDotPairs], v[kDotPairs];
+#pragma unroll
+    for (int j = 0; j < kDotPairs; ++j) {
+      u[j] = __ldg(a2 + q + j * stride);
+      v[j] = __ldg(b2 + q + j * stride);
+    }
+#pragma unroll
+    for (int j = 0; j < kDotPairs; ++j) acc[j] = add(add(acc[j], u[j].x, v[j].x), u[j].y, v[j].y);
+  }
+  for (; q < n2; q += stride) {
+    const double2 u = __ldg(a2 + q), v = __ldg(b2 + q);
+    acc[0] = add(add(acc[0], u.x, v.x), u.y, v.y);
+  }
+#pragma unroll 4
+  for (long long i = 2 * n2 + t; i < n; i += stride) acc[0] = add(acc[0], __ldg(a + i), __ldg(b + i));
+  const double s = block_sum((acc[0] + acc[1]) + (acc[2] + acc[3]), sh);
   if (threadIdx.x == 0) partial[blockIdx.x] = s;
 }
 
@@ -46,7 +85,11 @@ dot_final_kernel(const double* __restrict__ partial, int n, double* __restrict__
   release_next();
   wait_for_previous();
   double acc = 0.0;
-  for (int i = threadIdx.x; i < n; i += kDotTpb) acc += partial[i];
+#pragma unroll
+  for (int j = 0; j < SPB_VNEC_DOT_BLOCKS / kDotTpb; ++j) {
+    const int i = threadIdx.x + j * kDotTpb;
+    acc += i < n ? partial[i] : 0.0;
+  }
   const double s = block_sum(acc, sh);
   if (threadIdx.x == 0) out[0] = s;
 }
@@ -63,9 +106,12 @@ extern "C" SpB_Info SpB_VNEC_dot_ext(int64_t n, const double* d_a, const double*
     return SpB_FAILURE;
   }
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  return launch_chained(dot_partial_kernel, SPB_VNEC_DOT_BLOCKS, kDotTpb, 0, s, (long long)n, d_a, d_b, mode,
-                        d_partial) &&
-                 launch_chained(dot_final_kernel, 1, kDotTpb, 0, s, d_partial, SPB_VNEC_DOT_BLOCKS, d_out)
+  const bool vec = ((reinterpret_cast<uintptr_t>(d_a) | reinterpret_cast<uintptr_t>(d_b)) & 15) == 0;
+  const int blocks =
+      (int)std::min<long long>(SPB_VNEC_DOT_BLOCKS, std::max<long long>(1, (n + kDotBlockValues - 1) / kDotBlockValues));
+  return launch_chained(mode == 0 ? dot_partial_kernel<0> : dot_partial_kernel<1>, (unsigned)blocks, kDotTpb, 0, s,
+                        (long long)n, d_a, d_b, vec, d_partial) &&
+                 launch_chained(dot_final_kernel, 1, kDotTpb, 0, s, d_partial, blocks, d_out)
              ? SpB_SUCCESS
              : SpB_FAILURE;
 }
