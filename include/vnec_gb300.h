@@ -172,7 +172,8 @@ typedef struct {
                             descriptor, OpenSparseBLAS.h:62-72): x has n_rows entries,
                             y n_cols; any kernel, built on A's transpose */
   int host_parts;        /* sliced FP64 plans: host-vector calls run in this many parts so
-                            that y copies overlap the SpMV (0: 8, 1: one part) */
+                            that y copies overlap the SpMV (0: 4 where y is page-locked
+                            and of 12 MB at least, else one; 1: one part) */
   int column_deltas;     /* sliced: store the columns of one-row-per-lane groups as 16-bit
                             deltas where the gaps allow (0: on unless a hot-column window
                             is used, -1: off) */

@@ -95,6 +95,25 @@ struct DeviceBuffer {
   template <typename T> T* as() const { return static_cast<T*>(ptr); }
 };
 
+// Owning page-locked host allocation that kernels write to (`dev`).
+struct MappedBuffer {
+  void* host = nullptr;
+  void* dev = nullptr;
+  MappedBuffer() = default;
+  MappedBuffer(const MappedBuffer&) = delete;
+  MappedBuffer& operator=(const MappedBuffer&) = delete;
+  ~MappedBuffer() {
+    if (host) cudaFreeHost(host);
+  }
+  bool alloc(size_t n) {
+    if (!VNEC_CUDA(cudaHostAlloc(&host, n, cudaHostAllocMapped | cudaHostAllocPortable))) {
+      host = nullptr;
+      return false;
+    }
+    return VNEC_CUDA(cudaHostGetDevicePointer(&dev, host, 0));
+  }
+};
+
 // ---------------------------------------------------------------------------
 // Merge-path CSR kernels (the GPU counterpart of VNEC-L,
 // src/operation/src/spmv_vnec_L_for_mxv.c).

@@ -66,6 +66,7 @@ struct Plan {
   int device = 0;
   cudaStream_t own_stream = nullptr;
   DeviceBuffer dx, dy;  // staging for host-vector calls
+  MappedBuffer hy;      // y of short host-vector calls, written by the kernels (run_host)
   // The public handle carries NULL-filled per-partition pointer arrays
   // (Build_VNEC_S_* / Build_VNEC_D_*) that the release must free.
   bool pub_part_arrays = false;

@@ -30,6 +30,7 @@ struct SlicedPlan final : Plan {
     int64_t h0, h1;                  // heavy long rows (SlicedMatrix::long_heavy) of the part
   };
   std::vector<Part> parts;
+  bool parts_asked = false;  // by the host_parts option: every host call is split
   // Each part runs on its own stream, with stream priorities falling from the
   // first part to the last: all parts are launched together once x is on the
   // device, the block scheduler serves earlier parts first, so parts finish in
@@ -94,8 +95,25 @@ struct SlicedPlan final : Plan {
     }
     return true;
   }
+  // By default a call is split only where that pays: y page-locked, so that its
+  // copies run beside the kernels (a copy to pageable memory holds up the next
+  // part's launch: 200,000 rows 71 us whole, 144 in 8 parts; 16 M rows 1.86
+  // against 2.05 ms), and of 12 MB at least (page-locked, whole against 4 and 8
+  // parts: 200,000 rows 47, 63 and 62 us; 1.6 M 204, 197, 208; 16 M 1739, 1440,
+  // 1461).
+  bool split_pays(const void* h_y) const {
+    if (parts_asked) return true;
+    if ((type == SpB_FP64 ? 8 : 4) * n_rows < ((int64_t)12 << 20)) return false;
+    cudaPointerAttributes at{};
+    if (cudaPointerGetAttributes(&at, h_y) != cudaSuccess) {
+      cudaGetLastError();
+      return false;
+    }
+    return at.type == cudaMemoryTypeHost;
+  }
   bool run_host(const void* h_x, void* h_y) override {
-    if (mx.precision != kPrecFP64 || m.vpe != 1 || parts.size() < 2 || profiling) return Plan::run_host(h_x, h_y);
+    if (mx.precision != kPrecFP64 || m.vpe != 1 || parts.size() < 2 || profiling || !split_pays(h_y))
+      return Plan::run_host(h_x, h_y);
     std::lock_guard<std::mutex> g(host_mu);
     if (!drain_pipe()) return false;
     const size_t vb = type == SpB_FP64 ? 8 : 4;
@@ -534,9 +552,10 @@ std::unique_ptr<Plan> upload(std::unique_ptr<SlicedPlan> p, SlicedHost* h, int v
   const int ipt = opts ? opts->items_per_thread : 0;
   m.unroll = (ipt == 4 || ipt == 8 || ipt == 12 || ipt == 16) ? ipt : 12;
   if ((ipt == 0 || ipt == -1) && m.vpe == 1 && !p->tune_unroll()) return nullptr;
-  // Parts for host-vector calls: about 8 groups of whole windows with equal
+  // Parts for host-vector calls: about 4 groups of whole windows with equal
   // entries (only plans that compute every row: no keep mask).
-  const int kParts = (opts && opts->host_parts > 0) ? std::min(opts->host_parts, 1024) : 8;
+  p->parts_asked = opts && opts->host_parts > 0;
+  const int kParts = p->parts_asked ? std::min(opts->host_parts, 1024) : 4;
   if (hv.num_windows > 1 && !keep_mask && kParts > 1) {
     const int64_t W = p->prm.window_rows;
     int64_t w0 = 0;
