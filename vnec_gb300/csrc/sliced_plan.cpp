@@ -308,6 +308,13 @@ void hot_first_order(const CsrView& v, int32_t n_cols, const void* val, int vb, 
 constexpr int64_t kHotDefault = 32768;
 constexpr int64_t kHotDefaultX32 = 524288;
 constexpr double kHotMinCover = 0.05;
+// Below 2^20 columns the plain kernels and the DF32 form build no default window:
+// x (under 8 MB) is served well enough without, and the window costs a gather
+// launch per call.  R-MAT, degree 16, us with and without, FP64: 2^18 26.9 and
+// 24.3, 2^19 34.8 and 34.3, 2^20 57.8 and 59.5; FP32 type 21.3 and 17.4, 28.7 and
+// 27.2, 47.5 and 51.0.  The FP32 and BF16 forms keep theirs at every size: it
+// orders a row's entries, and so how its FP32 sums round.
+constexpr int64_t kHotMinCols = (int64_t)1 << 20;
 int64_t hot_window(const SpB_VNEC_options_ext* opts, double* min_cover) {
   *min_cover = 0.0;
   if (opts && opts->hot_columns < 0) return 0;
@@ -650,8 +657,9 @@ std::unique_ptr<Plan> build_sliced(const CsrView& v, const SpB_VNEC_options_ext*
   const bool x32 = prec == kPrecFP32 || prec == kPrecBF16;
   const bool default_window = min_cover > 0.0;  // no explicit hot_columns option
   bool have_hot = false;
+  const bool too_short = default_window && !x32 && v.n_cols < kHotMinCols;
   if (default_window && x32) have_hot = choose_hot(v, kHotDefaultX32, min_cover, &p->hot_host, &mapped);
-  if (!have_hot) have_hot = choose_hot(v, want_hot, min_cover, &p->hot_host, &mapped);
+  if (!have_hot && !too_short) have_hot = choose_hot(v, want_hot, min_cover, &p->hot_host, &mapped);
   if (have_hot) {
     cols = mapped.data();
     cols64 = nullptr;
