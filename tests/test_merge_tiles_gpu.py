@@ -1,5 +1,5 @@
 """The merge-path tile kernel at the edges of its threads and tiles: rows that
-end on, before and after a thread's 8 nonzeros and a tile's 896 items, rows of
+end on, before and after a thread's 8 nonzeros and a tile of 896, 1,016 or 2,040 items, rows of
 many threads and of many tiles, runs of empty rows, and caller arrays without
 the 32-byte alignment that its vector loads use."""
 from __future__ import annotations
@@ -17,7 +17,7 @@ LENGTHS = {
     "one": [1] * 3000,
     "thread": [7, 8, 9, 15, 16, 17, 1] * 300,
     "walk": [31, 32, 33, 40, 41, 200, 3] * 60,  # rows of up to, and past, four threads
-    "tile": [894, 895, 896, 897, 1, 888, 0, 7] * 5,
+    "tile": [894, 895, 896, 897, 1, 888, 0, 7, 1014, 1015, 1016, 1017, 2039, 2040, 2041] * 5,
     "hub": [0, 5, 20000, 0, 0, 3, 4481, 2] + [4] * 500 + [9000],
     "empty_runs": ([0] * 2000 + [3, 0, 12]) * 3 + [0] * 1500,
 }

@@ -120,10 +120,14 @@ struct MappedBuffer {
 // ---------------------------------------------------------------------------
 
 // Tile shape of the merge-path kernels: threads per CTA x merge items per thread.
+// The tile kernel gives a thread kMpPlaces nonzeros, and needs one thread's more
+// than a tile holds (mp_kernels.cu): a shape of kMpPlaces items per thread is the
+// tile that fills its threads.
+constexpr int kMpPlaces = 8;
 struct MpShape {
   int tpb = 256;
   int ipt = 7;
-  int64_t items_per_tile() const { return (int64_t)tpb * ipt; }
+  constexpr int64_t items_per_tile() const { return (int64_t)(ipt == kMpPlaces ? tpb - 1 : tpb) * ipt; }
 };
 
 // Value/accumulation forms of the merge-path kernel.

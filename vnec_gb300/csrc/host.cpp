@@ -484,11 +484,15 @@ std::unique_ptr<Plan> build_merge_path(const CsrView& v, const SpB_VNEC_options_
                  (req_stages >= 2 || req_arith == SpB_VNEC_ARITH_DF32 || other_shape);
   if (opts && opts->threads_per_block) sh.tpb = opts->threads_per_block;
   if (opts && opts->items_per_thread) sh.ipt = opts->items_per_thread;
-  // The default tile: small CTAs overlap the phases of a tile best (against
-  // 256 x 7: R-MAT 2^22 361 -> 293 us, 27-point stencil 120^3 234 -> 172).
-  if (!p->pipelined && !(opts && (opts->threads_per_block || opts->items_per_thread))) sh.tpb = 128;
+  // The default tile (both sides measured in mp_kernels.cu).
+  const bool default_tile = !p->pipelined && !(opts && (opts->threads_per_block || opts->items_per_thread));
+  if (default_tile) {
+    sh.tpb = 128;
+    sh.ipt = kMpPlaces;
+  }
   const int stages = req_stages >= 2 ? req_stages : 2;
-  if (p->pipelined ? mp2_smem(sh.tpb, sh.ipt, stages) == 0 : !shape_supported(sh.tpb, sh.ipt)) {
+  if (p->pipelined ? mp2_smem(sh.tpb, sh.ipt, stages) == 0
+                   : !default_tile && !shape_supported(sh.tpb, sh.ipt)) {
     set_error(p->pipelined ? "unsupported pipelined tile shape (256x7 s2/s3, 256x12 s2, 128x12 s3, 512x5 s2)"
                            : "unsupported merge-path tile shape (threads 128/256, items 4/7/10)");
     return nullptr;

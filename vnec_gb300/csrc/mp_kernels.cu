@@ -36,7 +36,10 @@
 // the FP32 type 193 and 102.  FP64 pipe 60% busy, L1 65%, L2 53 to 68%: no one
 // unit binds, the phases of a tile do.  Small CTAs overlap them best: tiles of
 // 128 x 7 items (one thread per 8 places) against 256 x 7 are 7 to 20% faster,
-// 16 nonzeros a thread up to 15% slower on power-law rows.
+// 16 nonzeros a thread up to 15% slower on power-law rows.  The default tile of
+// 1,016 items gives all of 128 threads their 8 places, where 896 left 15 idle:
+// 277 -> 267 and 180 -> 155 (64 threads, 504 items: 288 and 177; 96, 760: 264
+// and 161).
 
 #include <cuda_runtime.h>
 
@@ -112,7 +115,7 @@ template <int N> __device__ __forceinline__ void load_items(const int32_t* p, in
 }
 
 constexpr unsigned kNoRow = 0xffffu;  // slot of a nonzero that ends no row
-constexpr int E = 8;                  // nonzeros per thread
+constexpr int E = kMpPlaces;          // nonzeros per thread
 
 // Threads of a tile of `items` merge items: E nonzeros each, and one thread
 // more because the tile's first nonzero may lie inside its thread's E.
@@ -394,7 +397,7 @@ bool mp_spmv(const MpMatrix& m, MpForm form, const void* x, void* y, cudaStream_
 // allocator (the library could not obtain more), and latency-critical loops
 // in which a cudaMalloc/cudaFree and the device synchronisation it implies
 // are not acceptable.  For them this entry point runs the FP64 merge-path
-// kernel (256 threads x 7 merge items per tile) on CSR arrays the caller
+// kernel (256 threads, 2,040 merge items per tile) on CSR arrays the caller
 // already holds in device memory, and keeps its scratch — the merge
 // coordinates of each tile and each tile's carry-out — in the fixed array
 // below, which every device that loads this library holds until the process
@@ -403,11 +406,13 @@ bool mp_spmv(const MpMatrix& m, MpForm form, const void* x, void* y, cudaStream_
 namespace vnec {
 namespace {
 
-constexpr int kNaTpb = 256, kNaIpt = 7;
-// Scratch capacity: 2^18 tiles of 1,792 merge items, i.e. n_rows + nnz <=
-// 469,762,048; 5,242,888 bytes.
+constexpr MpShape kNaShape{256, kMpPlaces};
+// Scratch capacity: 2^18 tiles, 5,242,888 bytes.  The accepted size, n_rows + nnz
+// <= 469,762,048, takes 230,276 of them.
 constexpr long long kNaMaxTiles = 1LL << 18;
-constexpr long long kNaMaxItems = kNaMaxTiles * kNaTpb * kNaIpt;  // 469,762,048
+constexpr long long kNaMaxItems = 469762048;
+static_assert((kNaMaxItems + kNaShape.items_per_tile() - 1) / kNaShape.items_per_tile() <= kNaMaxTiles,
+              "the scratch holds every accepted size");
 constexpr size_t kNaTileRowOff = 0;
 constexpr size_t kNaTileNzOff = kNaTileRowOff + 4 * (kNaMaxTiles + 1);
 constexpr size_t kNaCarryRowOff = kNaTileNzOff + 4 * (kNaMaxTiles + 1);
@@ -497,7 +502,7 @@ extern "C" SpB_Info SpB_mxv_csr_noalloc_ext(int64_t n_rows, int64_t n_cols, int6
     set_error("SpB_mxv_csr_noalloc_ext: negative size");
     return SpB_FAILURE;
   }
-  const long long ipc = (long long)kNaTpb * kNaIpt;
+  const long long ipc = kNaShape.items_per_tile();
   // Each size is checked on its own before the sum is formed, so huge
   // arguments cannot overflow it.
   if (n_rows > kNaMaxItems || nnz > kNaMaxItems || n_rows + nnz > kNaMaxItems) {
@@ -530,8 +535,7 @@ extern "C" SpB_Info SpB_mxv_csr_noalloc_ext(int64_t n_rows, int64_t n_cols, int6
   m.carry_row = scratch + kNaCarryRowOff;
   m.carry_val = scratch + kNaCarryValOff;
   m.num_tiles = tiles;
-  m.shape.tpb = kNaTpb;
-  m.shape.ipt = kNaIpt;
+  m.shape = kNaShape;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   // Every scratch word a launch reads is written earlier in the same call
   // (coordinates by the partition kernel, carries by the tile kernel), so

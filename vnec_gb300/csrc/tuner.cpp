@@ -18,7 +18,7 @@ namespace vnec {
 namespace {
 
 // Merge-path configurations by items per thread: 4 and 7 run the tile kernel
-// (256 x 4, and 128 x 7, the tile of a default L plan), 12 the pipelined kernel
+// (256 x 4, and the tile of a default L plan), 12 the pipelined kernel
 // with 256 threads and two stages.  Warp-task configurations:
 // long-row chunk x dense-block fill threshold (1: every row with a block goes
 // dense, 1001: every row sliced).
@@ -101,8 +101,8 @@ SpB_VNEC_options_ext config_options(int i, const SpB_VNEC_options_ext* base) {
   const TuneConfig& c = kConfigs[i];
   o.kernel = c.kernel;
   if (c.kernel == SpB_VNEC_KERNEL_L) {
-    o.threads_per_block = c.chunk == 7 ? 128 : 256;
-    o.items_per_thread = c.chunk;
+    o.threads_per_block = c.chunk == 7 ? 0 : 256;
+    o.items_per_thread = c.chunk == 7 ? 0 : c.chunk;
     o.pipeline_stages = c.chunk == 12 ? 2 : 1;
   } else {
     o.threads_per_block = 0;
