@@ -161,7 +161,7 @@ enum SlicedPrecision : int { kPrecFP64 = 0, kPrecFP32 = 1, kPrecBF16 = 2, kPrecD
 struct SlicedMixed {
   int precision = kPrecFP64;
   void* xbuf = nullptr;                    // n_cols converted x: float (FP32/BF16) or float2 (DF32)
-  int* flag = nullptr;                     // DF32: x outside the split range this call
+  int* flag = nullptr;                     // DF32: [0] x outside the split range this call, [1] guard blocks done
   const signed char* row_scale = nullptr;  // BF16: power-of-two exponent per row slot
   const signed char* chunk_scale = nullptr;  // BF16: exponent per chunk
   const float2* val_split = nullptr;         // DF32: values as FP32 (hi, lo) truncation-split pairs
@@ -169,15 +169,25 @@ struct SlicedMixed {
 bool sliced_mixed_spmv(const SlicedMatrix& m, const SlicedMixed& mx, const double* x, double* y, cudaStream_t s,
                        cudaEvent_t* events = nullptr);
 // FP64 sliced kernel that only runs when *flag != 0 (DF32 fallback).
-bool sliced_guard_f64(const SlicedMatrix& m, const double* x, double* y, const int* flag, cudaStream_t s);
+bool sliced_guard_f64(const SlicedMatrix& m, const double* x, double* y, int* flag, cudaStream_t s);
 // FP64 -> FP32 round-to-nearest-even of n values on stream s (one launch).
 bool round_to_f32(const double* x, float* x32, long long n, cudaStream_t s);
 // Truncation split of n FP64 values into FP32 (hi, lo) pairs; sets *flag when a
 // nonzero value lies outside [2^-40, 2^41) (the caller clears it).
 bool split_to_df32(const double* x, float2* xs, long long n, int* flag, cudaStream_t s);
+// Small plans without a hot-column window or long rows gather FP64 x and convert
+// it at each gather instead of in a launch of its own first: that launch costs
+// about 2 us, the conversions 16 FP64-pipe cycles per 32 nonzeros.  FP32 form,
+// converted first -> at the gather: 100,000 nonzeros 7.5 -> 5.8 us (random
+// columns), 400,000 9.1 -> 8.1 (random) and 8.2 -> 7.0 (band of 33); a million
+// 9.8 -> 9.1 (random) but 13.8 -> 14.8 (band), two million 15.2 -> 17.7 (band),
+// so the line lies at 2^19.  Long rows (a lane's serial chain) keep the launch:
+// 400,000 nonzeros in log-normal rows 10.7 us with it, 13.6 without.
+constexpr int64_t kDirectNnz = (int64_t)1 << 19;
+inline bool sliced_mixed_direct(const SlicedMatrix& m) { return m.hot == 0 && m.num_long == 0 && m.nnz <= kDirectNnz; }
 inline int sliced_mixed_launches(const SlicedMatrix& m, int precision) {
-  return 2 + (precision == kPrecDF32 ? 1 : 0) + (m.num_long > 0 || precision == kPrecDF32 ? 1 : 0) +
-         (precision == kPrecDF32 && m.hot > 0 ? 1 : 0);
+  return (sliced_mixed_direct(m) ? 1 : 2) + (precision == kPrecDF32 ? (m.hot > 0 ? 2 : 1) : 0) +
+         (m.num_long > 0 ? 1 : 0);
 }
 inline FixupGrid fixup_grid(const SlicedMatrix& m, int threads) {
   const int64_t light = (m.num_long + threads - 1) / threads;

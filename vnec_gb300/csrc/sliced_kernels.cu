@@ -373,10 +373,11 @@ sliced_kernel(const SlicedTask* __restrict__ tasks, long long num_tasks, const V
 
 // FP64 recompute of a DF32 call whose x left the split range: a small grid of
 // warps striding the task list, so that the launch costs next to nothing in
-// the usual case (flag clear: every block returns at once).
+// the usual case (flag clear: every block returns at once).  The last block to
+// finish clears the flag, guard[0], for the next call; guard[1] counts them.
 template <bool HOT>
 __global__ void __launch_bounds__(kWarpsPerBlock * 32)
-sliced_guard_kernel(const int* __restrict__ guard, const SlicedTask* __restrict__ tasks, long long num_tasks,
+sliced_guard_kernel(int* guard, const SlicedTask* __restrict__ tasks, long long num_tasks,
                     const double* __restrict__ val, const int32_t* __restrict__ col,
                     const int32_t* __restrict__ rowid, const double* __restrict__ x, double* y,
                     double* __restrict__ chunk_sum, const double* __restrict__ xh, int ncols,
@@ -389,6 +390,11 @@ sliced_guard_kernel(const int* __restrict__ guard, const SlicedTask* __restrict_
   for (long long w = (long long)blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5); w < num_tasks; w += stride)
     sliced_task<double, 8, 0, HOT, false>(w, threadIdx.x & 31, tasks, val, col, rowid, x, y, chunk_sum, xh, ncols,
                                           ep, col16, first);
+  __syncthreads();
+  if (threadIdx.x == 0 && atomicAdd(guard + 1, 1) == (int)gridDim.x - 1) {
+    atomicExch(guard + 1, 0);
+    atomicExch(guard, 0);
+  }
 }
 
 template <typename V, bool EPI = false>
@@ -545,7 +551,7 @@ bool launch(const SlicedMatrix& m, const void* x, void* y, cudaStream_t s, cudaE
 
 }  // namespace
 
-bool sliced_guard_f64(const SlicedMatrix& m, const double* x, double* y, const int* flag, cudaStream_t s) {
+bool sliced_guard_f64(const SlicedMatrix& m, const double* x, double* y, int* flag, cudaStream_t s) {
   // The guard only runs for DF32 plans, whose FP64 values sit in m.val and
   // whose hot columns (if any) are served from x directly through hot_cols.
   int dev = 0, sms = 0;

@@ -13,12 +13,13 @@
 //          accumulation in FP32 (double-float), FP64 reductions — FP64-level
 //          accuracy on the FP32 pipe.  An x outside the split range raises a
 //          flag: the DF32 launch then returns at once and a guard launch of
-//          the FP64 sliced kernel computes the call.
+//          the FP64 sliced kernel computes the call and clears the flag.
 //
 // x conversion kernels: f64 -> f32 with round-to-nearest-even written from
 // the IEEE-754 definition in integer arithmetic (no FP64 instructions: the
 // FP64 pipe of GB300 converts at about 0.28 G/s per SM group), and the
-// truncation split f64 -> (hi, lo) used by DF32.
+// truncation split f64 -> (hi, lo) used by DF32.  Small plans have no
+// conversion launch (sliced_mixed_direct).
 
 #include <cuda_runtime.h>
 
@@ -171,6 +172,7 @@ __global__ void x_split_kernel(const double* __restrict__ x, float2* __restrict_
 }
 
 struct CodecF32 {
+  static constexpr bool kDirect = false;
   using Val = float;
   using Acc = float;
   __device__ static const void* at(const void* xs, int c) { return static_cast<const float*>(xs) + c; }
@@ -182,6 +184,7 @@ struct CodecF32 {
 };
 
 struct CodecBF16 {
+  static constexpr bool kDirect = false;
   using Val = unsigned short;
   using Acc = float;
   __device__ static const void* at(const void* xs, int c) { return static_cast<const float*>(xs) + c; }
@@ -193,6 +196,7 @@ struct CodecBF16 {
 };
 
 struct CodecDF32 {
+  static constexpr bool kDirect = false;
   using Val = float2;  // (hi, lo) split at plan build (the range was checked there)
   using Acc = DF;
   __device__ static const void* at(const void* xs, int c) { return static_cast<const float2*>(xs) + c; }
@@ -203,6 +207,47 @@ struct CodecDF32 {
   }
   __device__ static double to_f64(Acc a) { return df_to_f64(a); }
 };
+
+// The same forms on FP64 x (sliced_mixed_direct): x is rounded or split at each
+// gather, with the bits of the converted copy.  Rounding takes the FP64 pipe
+// (16 cycles a warp), which the latency of a small plan hides.
+struct CodecF32Direct : CodecF32 {
+  static constexpr bool kDirect = true;
+  __device__ static const void* at(const void* xs, int c) { return static_cast<const double*>(xs) + c; }
+  __device__ static Acc mac(Acc a, Val v, const void* xs, int c) {
+    return fmaf(v, __double2float_rn(__ldg(static_cast<const double*>(xs) + c)), a);
+  }
+};
+struct CodecBF16Direct : CodecBF16 {
+  static constexpr bool kDirect = true;
+  __device__ static const void* at(const void* xs, int c) { return static_cast<const double*>(xs) + c; }
+  __device__ static Acc mac(Acc a, Val v, const void* xs, int c) {
+    return fmaf(__uint_as_float(static_cast<unsigned>(v) << 16),
+                __double2float_rn(__ldg(static_cast<const double*>(xs) + c)), a);
+  }
+};
+struct CodecDF32Direct : CodecDF32 {
+  static constexpr bool kDirect = true;
+  struct Acc {
+    DF sum;
+    bool bad;  // met an x outside the split range
+  };
+  __device__ static const void* at(const void* xs, int c) { return static_cast<const double*>(xs) + c; }
+  __device__ static Acc zero() { return Acc{DF{0.0f, 0.0f}, false}; }
+  __device__ static Acc mac(Acc a, Val v, const void* xs, int c) {
+    float h, l;
+    const bool ok = df_split(__ldg(static_cast<const double*>(xs) + c), h, l);
+    return Acc{df_mac(a.sum, v.x, v.y, h, l), a.bad || !ok};
+  }
+  __device__ static double to_f64(const Acc& a) { return df_to_f64(a.sum); }
+};
+
+// A lane's sum as FP64; DF32 on FP64 x raises the flag for the guard launch.
+template <class C> __device__ __forceinline__ double finish(const typename C::Acc& a, int* flag) {
+  if constexpr (std::is_same<C, CodecDF32Direct>::value)
+    if (a.bad) atomicExch(flag, 1);
+  return C::to_f64(a);
+}
 
 template <typename T> __device__ __forceinline__ T ld_stream(const T* p) { return __ldcs(p); }
 template <> __device__ __forceinline__ unsigned short ld_stream<unsigned short>(const unsigned short* p) {
@@ -259,7 +304,7 @@ __global__ void __launch_bounds__(kWarps * 32)
 sliced_mixed_kernel(const SlicedTask* __restrict__ tasks, long long num_tasks, const typename C::Val* __restrict__ val,
                     const int32_t* __restrict__ col, const int32_t* __restrict__ rowid, const void* __restrict__ xs,
                     double* __restrict__ y, double* __restrict__ chunk_sum, const signed char* __restrict__ row_scale,
-                    const signed char* __restrict__ chunk_scale, const int* __restrict__ flag,
+                    const signed char* __restrict__ chunk_scale, int* flag,
                     const uint16_t* __restrict__ col16, const int32_t* __restrict__ first,
                     const uint16_t* __restrict__ pat16, SlicedPrefetch pf) {
   const long long w = ((long long)blockIdx.x * kWarps) + (threadIdx.x >> 5);
@@ -365,7 +410,7 @@ sliced_mixed_kernel(const SlicedTask* __restrict__ tasks, long long num_tasks, c
       }
     }
     if (lane < nrows) {
-      const double s = C::to_f64(acc);
+      const double s = finish<C>(acc, flag);
       y[rowid[row_base + lane]] = row_scale ? scale2(s, row_scale[row_base + lane]) : s;
     }
     return;
@@ -412,7 +457,7 @@ sliced_mixed_kernel(const SlicedTask* __restrict__ tasks, long long num_tasks, c
         acc = C::mac(acc, ld_stream(vp + k * 32), xs, c);
       }
       if (lane < nrows) {
-        const double s = C::to_f64(acc);
+        const double s = finish<C>(acc, flag);
         y[rowid[row_base + lane]] = row_scale ? scale2(s, row_scale[row_base + lane]) : s;
       }
       return;
@@ -455,7 +500,7 @@ sliced_mixed_kernel(const SlicedTask* __restrict__ tasks, long long num_tasks, c
           acc = C::mac(acc, tv[t], xs, c);
         }
       if (lane < nrows) {
-        const double s = C::to_f64(acc);
+        const double s = finish<C>(acc, flag);
         y[row] = row_scale ? scale2(s, row_scale[row_base + lane]) : s;
       }
       return;
@@ -480,7 +525,7 @@ sliced_mixed_kernel(const SlicedTask* __restrict__ tasks, long long num_tasks, c
       acc = C::mac(acc, ld_stream(vp + k * 32), xs, c);
     }
     if (lane < nrows) {
-      const double s = C::to_f64(acc);
+      const double s = finish<C>(acc, flag);
       y[rowid[row_base + lane]] = row_scale ? scale2(s, row_scale[row_base + lane]) : s;
     }
     return;
@@ -558,7 +603,7 @@ sliced_mixed_kernel(const SlicedTask* __restrict__ tasks, long long num_tasks, c
     for (int u = 0; u < U; ++u) acc = C::mac(acc, v[u], xs, c[u]);
   }
   for (; k < steps; ++k) acc = C::mac(acc, ld_stream(vp + k * 32), xs, __ldcs(cp + k * 32));
-  double s = C::to_f64(acc);
+  double s = finish<C>(acc, flag);
   for (int off = (1 << vwl) >> 1; off > 0; off >>= 1) s += __shfl_xor_sync(kFull, s, off);
   if (kind == kSlicedChunk) {
     if (lane == 0) chunk_sum[row_base] = chunk_scale ? scale2(s, chunk_scale[row_base]) : s;
@@ -572,23 +617,16 @@ sliced_mixed_kernel(const SlicedTask* __restrict__ tasks, long long num_tasks, c
 __global__ void long_fixup_f64(const int32_t* __restrict__ long_row, const int32_t* __restrict__ long_first,
                                const int32_t* __restrict__ long_heavy, long long num_long, long long num_heavy,
                                long long heavy_sub, unsigned light_blocks, const double* __restrict__ chunk_sum,
-                               double* __restrict__ y, int* flag) {
+                               double* __restrict__ y) {
   release_next();
   wait_for_previous();
-  if (blockIdx.x == 0 && threadIdx.x == 0 && flag) *flag = 0;  // consumed: reset for the next call
   long_rows_fixup<double>(long_first, long_heavy, num_long, num_heavy, heavy_sub, light_blocks, chunk_sum,
                           [&](long long i, double s) { y[long_row[i]] = s; });
 }
 
-__global__ void reset_flag(int* flag) {
-  release_next();
-  wait_for_previous();
-  *flag = 0;
-}
-
 template <class C>
 bool launch_mixed(const SlicedMatrix& m, const SlicedMixed& mx, const void* xs, double* y, cudaStream_t s,
-                  const int* flag) {
+                  int* flag) {
   const long long grid = (m.num_tasks + kWarps - 1) / kWarps;
   if (grid > 0x7fffffffLL) {
     set_error("sliced: too many tasks for one launch");
@@ -605,10 +643,14 @@ bool launch_mixed(const SlicedMatrix& m, const SlicedMixed& mx, const void* xs, 
   auto pick_u = [&](auto run, auto sh) {
     constexpr int P = decltype(run)::value;
     constexpr bool SH = decltype(sh)::value;
-    return m.unroll == 4    ? sliced_mixed_kernel<C, 4, P, SH>
-           : m.unroll == 12 ? sliced_mixed_kernel<C, 12, P, SH>
-           : m.unroll == 16 ? sliced_mixed_kernel<C, 16, P, SH>
-                            : sliced_mixed_kernel<C, 8, P, SH>;
+    // Plans small enough for FP64 x have short tasks and run at most 8 steps.
+    if constexpr (C::kDirect)
+      return m.unroll == 4 ? sliced_mixed_kernel<C, 4, P, SH> : sliced_mixed_kernel<C, 8, P, SH>;
+    else
+      return m.unroll == 4    ? sliced_mixed_kernel<C, 4, P, SH>
+             : m.unroll == 12 ? sliced_mixed_kernel<C, 12, P, SH>
+             : m.unroll == 16 ? sliced_mixed_kernel<C, 16, P, SH>
+                              : sliced_mixed_kernel<C, 8, P, SH>;
   };
   auto pick = [&](auto run) {
     return m.pat16 ? pick_u(run, std::true_type{}) : pick_u(run, std::false_type{});
@@ -630,10 +672,12 @@ bool sliced_mixed_spmv(const SlicedMatrix& m, const SlicedMixed& mx, const doubl
   const int tb = 256;
   const long long nx = m.n_cols;
   const int xg = (int)std::min<long long>((nx + m.hot + tb - 1) / tb, 152LL * 16);
-  int* flag = nullptr;
-  if (nx > 0) {
+  // x is read while y is written only where the two do not overlap; in place, x is converted first.
+  const char *xb = reinterpret_cast<const char*>(x), *yb = reinterpret_cast<const char*>(y);
+  const bool direct = sliced_mixed_direct(m) && (xb + 8 * nx <= yb || yb + 8 * m.n_rows <= xb);
+  int* flag = mx.precision == kPrecDF32 ? mx.flag : nullptr;
+  if (nx > 0 && !direct) {
     if (mx.precision == kPrecDF32) {
-      flag = mx.flag;
       if (!launch_chained(x_split_kernel, (unsigned)xg, tb, 0, s, x, static_cast<float2*>(mx.xbuf), nx, mx.flag,
                           m.hot_cols, m.hot))
         return false;
@@ -645,9 +689,18 @@ bool sliced_mixed_spmv(const SlicedMatrix& m, const SlicedMixed& mx, const doubl
   if (m.num_tasks > 0) {
     bool ok = false;
     switch (mx.precision) {
-      case kPrecFP32: ok = launch_mixed<CodecF32>(m, mx, mx.xbuf, y, s, nullptr); break;
-      case kPrecBF16: ok = launch_mixed<CodecBF16>(m, mx, mx.xbuf, y, s, nullptr); break;
-      case kPrecDF32: ok = launch_mixed<CodecDF32>(m, mx, mx.xbuf, y, s, flag); break;
+      case kPrecFP32:
+        ok = direct ? launch_mixed<CodecF32Direct>(m, mx, x, y, s, nullptr)
+                    : launch_mixed<CodecF32>(m, mx, mx.xbuf, y, s, nullptr);
+        break;
+      case kPrecBF16:
+        ok = direct ? launch_mixed<CodecBF16Direct>(m, mx, x, y, s, nullptr)
+                    : launch_mixed<CodecBF16>(m, mx, mx.xbuf, y, s, nullptr);
+        break;
+      case kPrecDF32:
+        ok = direct ? launch_mixed<CodecDF32Direct>(m, mx, x, y, s, flag)
+                    : launch_mixed<CodecDF32>(m, mx, mx.xbuf, y, s, flag);
+        break;
       default: set_error("sliced: unknown precision form"); return false;
     }
     if (!ok) return false;
@@ -662,10 +715,8 @@ bool sliced_mixed_spmv(const SlicedMatrix& m, const SlicedMixed& mx, const doubl
     const FixupGrid g = fixup_grid(m, b);
     if (!launch_chained(long_fixup_f64, g.total, b, 0, s, m.long_row, m.long_first, m.long_heavy,
                         (long long)m.num_long, (long long)m.num_heavy, (long long)m.heavy_sub, g.light,
-                        static_cast<const double*>(m.chunk_sum), y, mx.precision == kPrecDF32 ? mx.flag : nullptr))
+                        static_cast<const double*>(m.chunk_sum), y))
       return false;
-  } else if (mx.precision == kPrecDF32 && !launch_chained(reset_flag, 1, 1, 0, s, mx.flag)) {
-    return false;
   }
   if (ev && !VNEC_CUDA(cudaEventRecord(ev[2], s))) return false;
   return true;
