@@ -83,3 +83,26 @@ def test_unaligned_caller_arrays(built, name, shift):
     assert rc == api.SpB_SUCCESS, api.last_error()
     torch.cuda.synchronize()
     _check(y.cpu().numpy(), m, x, 1e-12)
+
+
+@pytest.mark.parametrize("shape", [(128, 4), (0, 0), (256, 4), (128, 10), (256, 7), (256, 10)])
+@pytest.mark.parametrize("width", [8, 16, 23, 24, 25, 31, 32, 33, 255, 257])
+def test_carries_between_threads(built, width, shape):
+    """Rows on both sides of the longest one that threads carry by walking back
+    (24 nonzeros, and by alignment up to 32), in tiles of 3, 4, 5, 6, 8 and 11
+    warps; a NaN and an infinity stay in their rows."""
+    from vnec_gb300 import api
+
+    m, x = _matrix([width] * 700 + [1, width + 1, 0] * 50, np.float64, seed=width)
+    for row, v in ((3, np.nan), (350, np.inf)):
+        m.val[m.row_ptr[row] + width // 2] = v
+    p = api.Plan(m, kernel=api.KERNEL_L, pipeline_stages=1, threads_per_block=shape[0], items_per_thread=shape[1])
+    y = p.mxv_host(x)
+    p.free()
+    assert np.isnan(y[3]) and np.isinf(y[350])
+    rows = np.setdiff1d(np.arange(m.n_rows), [3, 350])
+    assert np.all(np.isfinite(y[rows]))
+    m.val[~np.isfinite(m.val)] = 0.0
+    y[[3, 350]] = [m.val[m.row_ptr[r]:m.row_ptr[r + 1]] @ x[m.col[m.row_ptr[r]:m.row_ptr[r + 1]]] for r in (3, 350)]
+    # At most 257 products, 257 x 2^-53 of the row's condition (2.9e-14).
+    _check(y, m, x, 1e-13)

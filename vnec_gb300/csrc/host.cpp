@@ -473,7 +473,7 @@ std::unique_ptr<Plan> build_merge_path(const CsrView& v, const SpB_VNEC_options_
   // by default): by two or more stages, by DF32 sums, or by a tile shape other
   // than 256 x 7, which only the pipelined kernel takes when no stage count is
   // given.  The tile kernel is 2 to 3x faster on every matrix family, from 10^5
-  // nonzeros (R-MAT 2^14: 17.6 -> 12.5 us) to 5 10^7 (2^22: 874 -> 293), and
+  // nonzeros (R-MAT 2^14: 17.6 -> 6.4 us) to 5 10^7 (2^22: 874 -> 240), and
   // sums in FP64 where the pipelined default took double-float pairs.
   constexpr int64_t kPipelineMaxNnz = (int64_t)1 << 26;
   const bool large = req_stages == 0 && v.nnz >= kPipelineMaxNnz;

@@ -19,27 +19,37 @@
 //      shared-memory read: no search and no merge walk, and the only FP64
 //      work per nonzero is its FMA (an FP64 operation takes the pipe of a
 //      whole warp for 16 cycles here, whichever lanes need it);
-//   3. carry: a thread whose segment starts inside a row adds the partial sums
-//      of the preceding threads that stopped in the same row, found by a
-//      segmented scan over the threads (warp shuffles plus one scan over the
-//      warp totals, log steps), then writes that row; the tile's own
-//      carry-out (partial of its last row) goes to a per-tile scratch slot;
+//   3. carry: a thread whose first row end closes a row that began in an
+//      earlier thread adds the partial sums (tails) of the threads in between.
+//      Where no row of the tile passes over more than two whole threads, every
+//      thread walks back over them.  Else one warp takes all the tile's tails:
+//      a lane sums those of four threads, a segmented scan joins the lanes, and
+//      the lane goes over its four again to write their rows.  Either way the
+//      carries take some 8 to 12 FP64 instructions of a warp next to the 32 of
+//      the FMAs.  The tile's own carry-out (partial of its last row) goes to a
+//      per-tile scratch slot;
 //   4. fix-up (second, tiny launch): rows spanning tiles receive the ordered
 //      sum of the carries of the tiles that stopped inside them — the
 //      counterpart of the reference's serial carry loop (:159-164).
 //
 // What bounds it: the x gathers' L1/L2 requests on power-law columns, as in
-// the sliced kernel, without its hot-column window.
-// Measured on GB300 (R-MAT 2^22, 49 M nonzeros; 27-point stencil 120^3; us a
-// call, against the kernels it replaced as the default: pipelined DF32 tiles,
-// whose shared-memory merge walk bound them): FP64 874 -> 293 and 455 -> 172;
-// the FP32 type 193 and 102.  FP64 pipe 60% busy, L1 65%, L2 53 to 68%: no one
-// unit binds, the phases of a tile do.  Small CTAs overlap them best: tiles of
-// 128 x 7 items (one thread per 8 places) against 256 x 7 are 7 to 20% faster,
-// 16 nonzeros a thread up to 15% slower on power-law rows.  The default tile of
-// 1,016 items gives all of 128 threads their 8 places, where 896 left 15 idle:
-// 277 -> 267 and 180 -> 155 (64 threads, 504 items: 288 and 177; 96, 760: 264
-// and 161).
+// the sliced kernel, without its hot-column window, and the FP64 pipe on the
+// others: no one unit is full, the phases of a tile do not overlap all the way.
+// Measured on GB300 (us a call, FP64 / the FP32 type): R-MAT 2^22, 49 M nonzeros,
+// 240 / 173; 27-point stencil 120^3 153 / 76; a million rows of 16, 75 / 63; 20,001
+// rows of 1,000, 74 / 42.  Against the pipelined DF32 tiles, whose shared-memory
+// merge walk bound them: R-MAT 874, stencil 455.
+// Carries: with every row of a warp walked by a lane, and rows past four
+// threads shared by the lanes, they took as many FP64 instructions as half the
+// nonzeros (28 a tile; FP64 pipe 62% busy): R-MAT 267 / 178, rows of 1,000 101 /
+// 47, rows of 16 79 / 64, stencil 155 / 81.  The one warp alone loses on short
+// rows (rows of 16: 84, of 4: 105 against 88 with the walk).  Walks over at most 1, 2,
+// 3 whole threads: stencil 156, 153, 164; rows of 16 79, 77, 77.
+// Tiles: small CTAs overlap the phases best: 128 x 7 items (one thread per 8
+// places) against 256 x 7 are 7 to 20% faster, 16 nonzeros a thread up to 15%
+// slower on power-law rows.  The default tile of 1,016 items gives all of 128
+// threads their 8 places (64 threads, 504 items: 8% slower on R-MAT; 96, 760: 1%
+// faster there, 4% slower on the stencil).
 
 #include <cuda_runtime.h>
 
@@ -122,9 +132,41 @@ constexpr int E = kMpPlaces;          // nonzeros per thread
 constexpr int tile_threads(int items) { return ((items + E - 1) / E + 1 + 31) / 32 * 32; }
 constexpr int kMaxTileThreads = tile_threads(256 * 10);
 
+constexpr int kReach = 2;  // whole threads without a row end that a walk back crosses at most
+constexpr int kRake = 4;   // warps of the default tile: threads whose carries one lane takes
+
+// kRake consecutive shared-memory values as vector loads.
+__device__ __forceinline__ void rake_load(const double* p, double (&v)[kRake]) {
+  const double2 a = reinterpret_cast<const double2*>(p)[0], b = reinterpret_cast<const double2*>(p)[1];
+  v[0] = a.x, v[1] = a.y, v[2] = b.x, v[3] = b.y;
+}
+__device__ __forceinline__ void rake_load(const float* p, float (&v)[kRake]) {
+  const float4 a = *reinterpret_cast<const float4*>(p);
+  v[0] = a.x, v[1] = a.y, v[2] = a.z, v[3] = a.w;
+}
+__device__ __forceinline__ void rake_load(const unsigned short* p, unsigned short (&v)[kRake]) {
+  const ushort4 a = *reinterpret_cast<const ushort4*>(p);
+  v[0] = a.x, v[1] = a.y, v[2] = a.z, v[3] = a.w;
+}
+
+// Sum over the lanes back to the nearest one with `ends` (its own value alone
+// where that is the lane itself).
+template <typename V> __device__ __forceinline__ V rake_scan(V sum, bool ends, int lane) {
+  constexpr unsigned kFull = 0xffffffffu;
+  const unsigned below = __ballot_sync(kFull, ends) & (kFull >> (31 - lane));
+  const int reach = below ? __clz(below) - (31 - lane) : lane;
+  const int longest = (int)__reduce_max_sync(kFull, (unsigned)reach);
+  for (int d = 1; d <= longest; d <<= 1) {
+    const V up = __shfl_up_sync(kFull, sum, d);
+    sum += d <= reach ? up : V(0);
+  }
+  return sum;
+}
+
 // One CTA per tile, of at most T threads with E nonzeros each; at least B CTAs
-// fit an SM.  Dynamic shared memory: a 16-bit slot per nonzero place, then each thread's head and tail sums.  `vec`: col and val
-// are 32-byte aligned.
+// fit an SM.  Dynamic shared memory: a 16-bit slot per nonzero place, then each
+// thread's tail and head sums and the row of its first row end.  `vec`: col and
+// val are 32-byte aligned.
 template <typename V, typename Off, int T, int B>
 __global__ void __launch_bounds__(T, B)
 mp_spmv_kernel(const Off* __restrict__ row_end, const int32_t* __restrict__ col, const V* __restrict__ val,
@@ -135,6 +177,7 @@ mp_spmv_kernel(const Off* __restrict__ row_end, const int32_t* __restrict__ col,
   extern __shared__ uint4 s_slots[];
   V* const s_tail = reinterpret_cast<V*>(s_slots + (E / 8) * blockDim.x);
   V* const s_head = s_tail + blockDim.x;
+  unsigned short* const s_first = reinterpret_cast<unsigned short*>(s_head + blockDim.x);
   const int tile = blockIdx.x;
   const int tid = threadIdx.x, lane = tid & 31;
   release_next();
@@ -197,65 +240,115 @@ mp_spmv_kernel(const Off* __restrict__ row_end, const int32_t* __restrict__ col,
     sw[4 * h + 2] = s4.z;
     sw[4 * h + 3] = s4.w;
   }
-  // The sum up to the thread's first row end goes to its head, what follows
-  // its last row end (everything, if no row ends here) to its tail; a row
-  // between two ends is complete.
-  V acc = V(0);
-  bool any = false;
+  // The sum up to the thread's first row end is its head, what follows its
+  // last row end (everything, if no row ends here) its tail; a row between two
+  // ends is complete.
+  V acc = V(0), head = V(0);
+  unsigned first = kNoRow;
 #pragma unroll
   for (int j = 0; j < E; ++j) {
     acc = fma_v<V>(v[j], xv[j], acc);  // outside the branch: one FP64 instruction for the whole warp
     const unsigned r = (sw[j >> 1] >> (16 * (j & 1))) & 0xffffu;
     if (r != kNoRow) {
-      if (any)
+      if (first != kNoRow) {
         y[x0 + r] = acc;
-      else
-        s_head[tid] = acc;
-      any = true;
+      } else {
+        head = acc;
+        first = r;
+      }
       acc = V(0);
     }
   }
   s_tail[tid] = acc;
-  __syncthreads();
+  s_head[tid] = head;
+  s_first[tid] = (unsigned short)first;
+  const unsigned open = __ballot_sync(kFull, first == kNoRow && q < end);
+  unsigned run = open;  // more than kReach threads in a row without a row end?
+#pragma unroll
+  for (int i = 1; i <= kReach; ++i) run &= open >> i;
 
-  // 3. rows that begin in an earlier thread than they end in, or at its edge:
-  // lane r adds the tails from the row's first thread on, then the head of its
-  // last.  Where that takes fewer FP64 instructions of the warp (the longest
-  // walk against kShare for each row past kWalk threads), the lanes share the
-  // longer rows instead.  "Row" nrows is what the tile leaves open: the carry.
-  constexpr int kWalk = 4, kShare = 6;
-  for (int r0 = tid - lane; r0 <= nrows; r0 += blockDim.x) {
-    const int r = r0 + lane;
-    int b = 0, e = 0;
-    bool mine = false;
-    if (r <= nrows) {
-      e = r < nrows ? (int)(row_end[x0 + r] - y0) + lead : end;
-      b = r ? (int)(row_end[x0 + r - 1] - y0) + lead : lead;
-      mine = e > b;
-      if (b == lead) b = 0;  // the zero places before the tile count as the first row's
-      mine = mine && (r == nrows || b <= (e - 1) / E * E);
+  // 3. carries between threads.  Rows of a few threads each: every thread
+  // walks back from its first row end.
+  if (!__syncthreads_or(run != 0)) {
+    const bool last = q < end && q + E >= end;
+    if (first != kNoRow || last) {
+      V s = first != kNoRow ? head : acc;
+      for (int t = tid - 1; t >= 0; --t) {
+        s += s_tail[t];
+        if (s_first[t] != kNoRow) break;
+      }
+      if (first != kNoRow) y[x0 + first] = s;
+      if (last) {
+        carry_row[tile] = x1;
+        carry_val[tile] = first != kNoRow ? acc : s;
+      }
     }
-    const int te = (e - 1) / E, t0 = b / E, t1 = r < nrows ? te : te + 1;  // tails t0 .. t1 - 1
-    const int span = mine ? t1 - t0 : 0;
-    const unsigned many = __ballot_sync(kFull, span > kWalk);
-    const int longest = (int)__reduce_max_sync(kFull, (unsigned)span);  // every lane takes part
-    const bool shared = span > kWalk && kWalk + kShare * __popc(many) < longest;
-    V s = V(0);
-    if (mine && !shared)
-      for (int t = t0; t < t1; ++t) s += s_tail[t];
-    for (unsigned m = __ballot_sync(kFull, shared); m; m &= m - 1) {
-      const int src = __ffs(m) - 1;
-      const int u0 = __shfl_sync(kFull, t0, src), u1 = __shfl_sync(kFull, t1, src);
-      V p = V(0);
-      for (int t = u0 + lane; t < u1; t += 32) p += s_tail[t];
-      for (int off = 16; off > 0; off >>= 1) p += __shfl_xor_sync(kFull, p, off);
-      if (lane == src) s = p;
-    }
-    if (r < nrows) {
-      if (mine) y[x0 + r] = t1 > t0 ? s + s_head[te] : s_head[te];
-    } else if (r == nrows) {
+    if (tid == 0 && end == lead) {
       carry_row[tile] = x1;
-      carry_val[tile] = s;
+      carry_val[tile] = V(0);
+    }
+    return;
+  }
+
+  // Longer rows: by one warp of the tile (not the same one in each); a lane
+  // takes the carries of K threads in a row.
+  const int warps = (int)(blockDim.x >> 5), turn = tile & 3;
+  if ((tid >> 5) != (turn < warps ? turn : 0)) return;
+  if (warps == kRake) {
+    // The default tile: everything a lane needs in a few vector loads.
+    V tail[kRake], head4[kRake];
+    unsigned short r4[kRake];
+    rake_load(s_tail + lane * kRake, tail);
+    rake_load(s_first + lane * kRake, r4);
+    rake_load(s_head + lane * kRake, head4);
+    bool ends = r4[0] != kNoRow;
+    V sum = tail[0];
+#pragma unroll
+    for (int k = 1; k < kRake; ++k) {
+      const bool f = r4[k] != kNoRow;
+      ends |= f;
+      sum = (f ? V(0) : sum) + tail[k];
+    }
+    sum = rake_scan(sum, ends, lane);
+    if (lane == 31) {
+      carry_row[tile] = x1;
+      carry_val[tile] = sum;
+    }
+    sum = __shfl_up_sync(kFull, sum, 1);
+    if (lane == 0) sum = V(0);
+#pragma unroll
+    for (int k = 0; k < kRake; ++k) {
+      const bool f = r4[k] != kNoRow;
+      sum += f ? head4[k] : tail[k];
+      if (f) {
+        y[x0 + r4[k]] = sum;
+        sum = tail[k];
+      }
+    }
+    return;
+  }
+  const int K = warps, t0 = lane * K;
+  bool ends = false;
+  V sum = V(0);
+  for (int k = 0; k < K; ++k) {
+    const bool f = s_first[t0 + k] != kNoRow;
+    ends |= f;
+    sum = (f ? V(0) : sum) + s_tail[t0 + k];
+  }
+  sum = rake_scan(sum, ends, lane);
+  if (lane == 31) {
+    carry_row[tile] = x1;
+    carry_val[tile] = sum;
+  }
+  sum = __shfl_up_sync(kFull, sum, 1);
+  if (lane == 0) sum = V(0);
+  for (int k = 0; k < K; ++k) {
+    const unsigned r = s_first[t0 + k];
+    const V tail = s_tail[t0 + k];
+    sum += r != kNoRow ? s_head[t0 + k] : tail;
+    if (r != kNoRow) {
+      y[x0 + r] = sum;
+      sum = tail;
     }
   }
 }
@@ -318,7 +411,7 @@ bool launch_tiles(const MpMatrix& m, int threads, const void* x, void* y, cudaSt
     return false;
   }
   const bool vec = ((reinterpret_cast<uintptr_t>(m.col) | reinterpret_cast<uintptr_t>(m.val)) & 31) == 0;
-  const size_t smem = (size_t)threads * (E * sizeof(unsigned short) + 2 * sizeof(V));
+  const size_t smem = (size_t)threads * ((E + 1) * sizeof(unsigned short) + 2 * sizeof(V));
   if (m.in_place)
     return launch_chained(kern, (unsigned)m.num_tiles, threads, smem, s, static_cast<const Off*>(m.row_end), m.col,
                           static_cast<const V*>(m.val), static_cast<const V*>(x), static_cast<V*>(y),
@@ -339,9 +432,9 @@ bool launch_mp(const MpMatrix& m, const void* x, void* y, cudaStream_t s, cudaEv
     set_error("merge-path: unsupported tile shape");
     return false;
   }
-  // 40 warps of an SM for FP64 (48 registers a thread), 64 for FP32: FP64 runs
-  // at 40 as at 48 (40 registers, which spill) or at 36, FP32 slows down by 7%
-  // at 48 warps and by 15% at 40 (R-MAT 2^22: 193, 207 and 225 us).
+  // 40 warps of an SM for FP64 (48 registers a thread), 64 for FP32: FP64 at 48
+  // (40 registers, which spill) is 6% faster to 13% slower, at 36 up to 12%
+  // slower; FP32 slows down by 7% at 48 warps and by 15% at 40.
   constexpr int kB = sizeof(V) == 8 ? 10 : 16;
   if (!(threads <= 128   ? launch_tiles<V, Off, 128, kB>(m, threads, x, y, s)
         : threads <= 256 ? launch_tiles<V, Off, 256, kB / 2>(m, threads, x, y, s)
