@@ -192,7 +192,8 @@ typedef struct {
                             integers (always done from 2^31 - 1 rows + nonzeros on) */
   int shared_patterns;   /* sliced plans: groups of rows with equal length and the
                             same column gaps (stencils, banded rows) read one copy of the gaps
-                            per group (0: on, -1: off; the sums are the same either way) */
+                            per group (0: where it pays, > 0: wherever they do, -1: off; the
+                            sums are the same either way) */
   int l2_prefetch;       /* sliced plans: each warp has the L2 prefetch the stored entries (values
                             and columns) this many entries past its own task's, and the task
                             metadata the same distance ahead, so that the tasks' loads meet

@@ -39,7 +39,7 @@ def test_shared_steps(built, width, form):
     for unroll in (4, 8, 12, 16):
         for lanes in (0, -1, 1):
             got = []
-            for shared in (0, -1):
+            for shared in (1, -1):
                 p = api.Plan(m, dtype=dtype, kernel=api.KERNEL_S, precision=prec, items_per_thread=unroll, max_steps=32,
                              shared_patterns=shared, lane_vectors=lanes)
                 z = torch.from_numpy(x[::-1].copy()).cuda()
@@ -50,3 +50,22 @@ def test_shared_steps(built, width, form):
             assert got[0][0].tobytes() == got[1][0].tobytes() and got[0][1].tobytes() == got[1][1].tobytes()
             assert got[0][2] < got[1][2]
             assert np.all(np.abs(got[0][0].astype(np.float64) - y_ref) <= tol * cond)
+
+
+@pytest.mark.parametrize("form,least", [("fp64", 14), ("fp32 type", 4), ("fp32", 2)])
+def test_default_rule(built, form, least):
+    """By default plain plans share patterns from 14 (FP64) or 4 (FP32 type) steps
+    on, the precision forms at every length; the bits are those of all and of none."""
+    from vnec_gb300 import api
+
+    dtype = np.float32 if form == "fp32 type" else np.float64
+    for width in (2, 3, 4, 5, 13, 14, 15):
+        m, x = _pattern(width, dtype)
+        got = {}
+        for shared in (-1, 0, 1):
+            p = api.Plan(m, dtype=dtype, kernel=api.KERNEL_S, precision=api.PREC_FP32 if form == "fp32" else api.PREC_FP64,
+                         max_steps=32, shared_patterns=shared, column_deltas=0)
+            got[shared] = (p.mxv_host(x).tobytes(), p.info().algorithmic_bytes)
+            p.free()
+        assert got[-1][0] == got[0][0] == got[1][0]
+        assert got[0][1] == got[1 if width >= least else -1][1] and got[1][1] < got[-1][1]

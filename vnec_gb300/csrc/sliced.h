@@ -96,6 +96,7 @@ struct SlicedParams {
   int hot = 0;                // hot-column window size (0: none)
   bool delta16 = false;       // 16-bit column deltas for VW = 1 groups whose rows allow it
   bool shared = false;        // delta16 layouts: also mark shared-pattern tasks (kSlicedShared)
+  int shared_min = 1;         // of at least this many steps
   // Optional secondary key of the row sort (rows of equal length in a window
   // are grouped in ascending key order), n_rows values, or null.
   const int32_t* row_key = nullptr;

@@ -246,7 +246,7 @@ SlicedHost* sliced_build(int64_t n_rows, int64_t /*n_cols*/, const int64_t* rp, 
           int meta = kSlicedDelta;
           // Shared pattern: every row has `steps` entries and the first row's
           // deltas (at most 32 steps: one lane per step holds the pattern).
-          bool shared = h->pat16 && nrows > 0 && t.steps <= 32 && t.base % 32 == 0;
+          bool shared = h->pat16 && nrows > 0 && t.steps >= prm.shared_min && t.steps <= 32 && t.base % 32 == 0;
           const int64_t b0 = shared ? begin(h->rowid[(size_t)t.row_base]) : 0;
           for (int g = 0; g < nrows && shared; ++g) {
             const int64_t b = begin(h->rowid[(size_t)(t.row_base + g)]);

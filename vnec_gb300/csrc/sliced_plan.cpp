@@ -676,6 +676,14 @@ std::unique_ptr<Plan> build_sliced(const CsrView& v, const SpB_VNEC_options_ext*
   // Shared-pattern tasks (the per-lane deltas stay stored: the DF32 form's FP64
   // guard and the cache-hint variants walk them).
   p->prm.shared = p->prm.delta16 && !(opts && opts->shared_patterns < 0);
+  // Plain plans only from 14 (FP64) or 4 (FP32 type) steps on: the offsets of a
+  // task come through shared memory before its first x, which short rows do not
+  // pay back there (the precision forms' values are narrower or their sums
+  // longer: they gain at every length).  Bands of 20 M nonzeros, without -> with
+  // shared patterns, FP64: 2 wide 100 -> 130 us, 5 56 -> 72, 8 44 -> 47, 11 44 ->
+  // 44, 15 43 -> 41, 20 43 -> 38, 27 46 -> 40; FP32 type: 3 wide 73 -> 66 (but 2 M
+  // nonzeros 7.3 -> 7.6), 5 45 -> 45, 11 27 -> 23, 27 26 -> 17.
+  if (prec == kPrecFP64 && !(opts && opts->shared_patterns > 0)) p->prm.shared_min = vb == 8 ? 14 : 4;
   SlicedHost* h = sliced_build(v.n_rows, v.n_cols, v.ptr, v.ptr64, cols, cols64, src_val, vb, p->prm, 1, keep);
   if (!h) {
     set_error("sliced format: more than 2^31 entries or row slots");
