@@ -68,6 +68,7 @@ struct SlicedMatrix {
   int cache_hints = 0;                  // load cache-hint variant (sliced_kernels.cu), 0 default
   int unroll = 8;                       // load steps in flight per lane: 4, 8, 12 or 16
   int vpe = 1;                          // values per entry: 1 (nonzeros) or 4 (dense blocks)
+  int longest = 0;                      // most steps of any task
   // Hot-column window: the `hot` most frequently used columns are relabelled
   // n_cols + slot in `col`, and each call gathers their x values into a dense
   // array (xhot for the FP64 kernel, the tail of the converted x for the

@@ -130,23 +130,26 @@ template <> struct Quad<float> {
   }
 };
 
-// One warp per task, kDenseAhead<V> blocks of a lane in flight: their columns and
-// values are loaded together (the values do not wait for the columns), then their
-// x, and the last round is predicated instead of taking its blocks one by one.
+// One warp per task, U blocks of a lane in flight: their columns and values are
+// loaded together (the values do not wait for the columns), then their x, and the
+// last round is predicated instead of taking its blocks one by one.  U is 2 where
+// no task has more than kDenseShort blocks a lane, else kDenseAhead<V>.
 // What bounds it: latency (a block's columns, then its x; DRAM 40% busy before),
-// and for FP64 the FP64 pipe on filled-up blocks.  FP32 blocks of 24 x 24, 500,003
-// rows: 18.6 -> 12.6 us (4, 5, 8 blocks ahead: 12.9, 13.9, 13.4); band of 65:
-// 12.6 -> 9.7; lognormal rows, mostly one nonzero a block: 71 -> 65 (6) but 74
-// with 4 or 8 (4 needs more registers there).  FP64 at 4: band of 65 23.2 -> 19.7,
-// stencil 100^3 67.7 -> 67.5 (2: 64.9, but 98 -> 104 on lognormal rows).
+// and for FP64 the FP64 pipe on filled-up blocks.  Against one block after the
+// other, us: FP32 blocks of 24 x 24, 500,003 rows, 18.6 -> 11.6 (U = 6 12.7); band
+// of 6, 3 M rows, FP64 49 -> 45 (4: 55), FP32 41 -> 22 (6: 35); stencil 100^3 68 -> 65
+// (4: 67) and 38 -> 31 (6: 32).  With longer tasks, where a chain of rounds ends the
+// call, U = 2 loses: lognormal rows FP64 108 (4) against 121, FP32 81 (6) against 89
+// (4 or 8: 74 against 65 at another size); 40,001 of them 34 against 49; 16 random
+// columns a row, FP64, 49 against 61; band of 129 43 against 46.
 template <typename V> constexpr int kDenseAhead = sizeof(V) == 8 ? 4 : 6;
+constexpr int kDenseShort = 10;
 
-template <typename V>
+template <typename V, int U>
 __global__ void __launch_bounds__(kWarpsPerBlock * 32)
 dense_block_kernel(const SlicedTask* __restrict__ tasks, long long num_tasks, const V* __restrict__ val,
                    const int32_t* __restrict__ col, const int32_t* __restrict__ rowid, const V* __restrict__ x,
                    int n_cols, V* __restrict__ y, V* __restrict__ chunk_sum) {
-  constexpr int U = kDenseAhead<V>;
   const long long w = ((long long)blockIdx.x * kWarpsPerBlock) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   release_next();
@@ -430,7 +433,8 @@ bool launch_dense(const SlicedMatrix& m, const void* x, void* y, cudaStream_t s)
     set_error("dense blocks: too many tasks for one launch");
     return false;
   }
-  return launch_chained(dense_block_kernel<V>, (unsigned)grid, kWarpsPerBlock * 32, 0, s, m.tasks, m.num_tasks,
+  const auto kern = m.longest <= kDenseShort ? dense_block_kernel<V, 2> : dense_block_kernel<V, kDenseAhead<V>>;
+  return launch_chained(kern, (unsigned)grid, kWarpsPerBlock * 32, 0, s, m.tasks, m.num_tasks,
                         static_cast<const V*>(m.val), m.col, m.rowid, static_cast<const V*>(x), (int)m.n_cols,
                         static_cast<V*>(y), static_cast<V*>(m.chunk_sum));
 }

@@ -515,6 +515,7 @@ std::unique_ptr<Plan> upload(std::unique_ptr<SlicedPlan> p, SlicedHost* h, int v
   m.vpe = hv.vpe;
   m.entries = hv.entries;
   m.num_tasks = hv.num_tasks;
+  for (int64_t t = 0; t < hv.num_tasks; ++t) m.longest = std::max<int>(m.longest, hv.tasks[t].steps);
   m.num_long = hv.num_long;
   m.num_chunks = hv.num_chunks;
   m.tasks = p->tasks.as<SlicedTask>();
