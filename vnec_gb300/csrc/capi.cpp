@@ -250,7 +250,7 @@ SpB_VNEC_type IRD_VNEC(const SpB_Matrix A, SpB_Type type) {
 // because the reference's harness sends every matrix of 3e6 rows or more to
 // VNEC-L (test_spmv_vnec.cpp:197,235-256), and at those sizes the merge-path
 // kernel is 2.5x slower than the selected plan on a power-law matrix (R-MAT
-// 2^24: 2.30 vs 0.92 ms).  A merge-path plan of any size stays available
+// 2^24: 1.29 vs 0.91 ms).  A merge-path plan of any size stays available
 // through SpB_VNEC_plan_ext with kernel SpB_VNEC_KERNEL_L.
 constexpr int64_t kBuildLSelectNnz = (int64_t)1 << 26;
 
