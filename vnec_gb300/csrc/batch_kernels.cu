@@ -81,27 +81,27 @@ template <bool WIDE, bool VEC, typename T, int R> __device__ __forceinline__ voi
   constexpr int bytes = R * (int)sizeof(T);
   if constexpr (!VEC) {
 #pragma unroll
-    for (int r = 0; r < R; ++r) v[r] = __ldg(p + r);
+    for (int r = 0; r < R; ++r) v[r] = ld_prev(p + r);
   } else if constexpr (WIDE && bytes >= 32) {
 #pragma unroll
     for (int i = 0; i < bytes / 32; ++i) {
       uint32_t w[8];
-      asm("ld.global.nc.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-          : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]), "=r"(w[4]), "=r"(w[5]), "=r"(w[6]), "=r"(w[7])
-          : "l"(reinterpret_cast<const char*>(p) + 32 * i));
+      asm volatile("ld.global.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                   : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]), "=r"(w[4]), "=r"(w[5]), "=r"(w[6]), "=r"(w[7])
+                   : "l"(reinterpret_cast<const char*>(p) + 32 * i));
       memcpy(reinterpret_cast<char*>(v) + 32 * i, w, 32);
     }
   } else if constexpr (bytes >= 16) {
 #pragma unroll
     for (int i = 0; i < bytes / 16; ++i) {
-      const int4 q = __ldg(reinterpret_cast<const int4*>(p) + i);
+      const int4 q = ld_prev(reinterpret_cast<const int4*>(p) + i);
       memcpy(reinterpret_cast<char*>(v) + 16 * i, &q, 16);
     }
   } else if constexpr (bytes == 8) {
-    const int2 q = __ldg(reinterpret_cast<const int2*>(p));
+    const int2 q = ld_prev(reinterpret_cast<const int2*>(p));
     memcpy(v, &q, 8);
   } else {
-    const int q = __ldg(reinterpret_cast<const int*>(p));
+    const int q = ld_prev(reinterpret_cast<const int*>(p));
     memcpy(v, &q, 4);
   }
 }
@@ -215,7 +215,7 @@ constexpr int kStageRounds = 4;
 // the right-hand sides: every slot's sums are those of TL = 0, bit for bit, but
 // fewer lanes read each column and value and X comes in wider loads.
 template <class Cd, int R, int U, bool STAGED, bool VEC, int TL = 0>
-__device__ __forceinline__ void run_tasks(const BatchArgs& a, const typename Cd::X* __restrict__ x) {
+__device__ __forceinline__ void run_tasks(const BatchArgs& a, const typename Cd::X* x) {
   static_assert(TL == 0 || (!STAGED && Cd::kAhead), "several tasks per warp run the fetch-ahead loop");
   using V = typename Cd::V;
   using X = typename Cd::X;
@@ -227,7 +227,7 @@ __device__ __forceinline__ void run_tasks(const BatchArgs& a, const typename Cd:
   const int slot = lane >> ll, sub = lane & ((1 << ll) - 1);
   const long long nw = (long long)gridDim.x * (blockDim.x >> 5);
   const V* __restrict__ val = static_cast<const V*>(a.val);
-  const X* __restrict__ xs = x + sub * R;
+  const X* xs = x + sub * R;
   for (long long w0 = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); w0 << TL < a.num_tasks;
        w0 += nw) {
     const long long t = (w0 << TL) + ((threadIdx.x & 31) >> (5 - TL));

@@ -18,12 +18,13 @@
 
 namespace vnec {
 
-// out(i, s) stores long row i's sum s.
+// out(i, s) stores long row i's sum s.  (The chunk sums are another kernel's
+// results: no __restrict__, launch.cuh.)
 template <typename V, typename Out>
 __device__ __forceinline__ void long_rows_fixup(const int32_t* __restrict__ long_first,
                                                 const int32_t* __restrict__ long_heavy, long long num_long,
                                                 long long num_heavy, long long heavy_sub, unsigned light_blocks,
-                                                const V* __restrict__ chunk_sum, Out out) {
+                                                const V* chunk_sum, Out out) {
   if (blockIdx.x < light_blocks) {
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= num_long) return;

@@ -36,7 +36,7 @@
 // the sliced kernel, without its hot-column window, and the FP64 pipe on the
 // others: no one unit is full, the phases of a tile do not overlap all the way.
 // Measured on GB300 (us a call, FP64 / the FP32 type): R-MAT 2^22, 49 M nonzeros,
-// 240 / 173; 27-point stencil 120^3 153 / 76; a million rows of 16, 75 / 63; 20,001
+// 242 / 175; 27-point stencil 120^3 153 / 76; a million rows of 16, 75 / 63; 20,001
 // rows of 1,000, 74 / 42.  Against the pipelined DF32 tiles, whose shared-memory
 // merge walk bound them: R-MAT 874, stencil 455.
 // Carries: with every row of a warp walked by a lane, and rows past four
@@ -170,9 +170,8 @@ template <typename V> __device__ __forceinline__ V rake_scan(V sum, bool ends, i
 template <typename V, typename Off, int T, int B>
 __global__ void __launch_bounds__(T, B)
 mp_spmv_kernel(const Off* __restrict__ row_end, const int32_t* __restrict__ col, const V* __restrict__ val,
-               const V* __restrict__ x, V* __restrict__ y, const Off* __restrict__ tile_row,
-               const Off* __restrict__ tile_nz, Off nnz, bool vec, Off* __restrict__ carry_row,
-               V* __restrict__ carry_val) {
+               const V* x, V* y, const Off* __restrict__ tile_row, const Off* __restrict__ tile_nz, Off nnz, bool vec,
+               Off* carry_row, V* carry_val) {
   constexpr unsigned kFull = 0xffffffffu;
   extern __shared__ uint4 s_slots[];
   V* const s_tail = reinterpret_cast<V*>(s_slots + (E / 8) * blockDim.x);
@@ -182,10 +181,9 @@ mp_spmv_kernel(const Off* __restrict__ row_end, const int32_t* __restrict__ col,
   const int tid = threadIdx.x, lane = tid & 31;
   release_next();
   const Off x0 = tile_row[tile], y0 = tile_nz[tile];
-  const Off x1 = tile_row[tile + 1], y1 = tile_nz[tile + 1];
-  const int nrows = (int)(x1 - x0);
+  const int nrows = (int)(tile_row[tile + 1] - x0);
   const int lead = (int)(y0 & (E - 1));   // places before the tile's first nonzero
-  const int end = lead + (int)(y1 - y0);  // one past its last
+  const int end = lead + (int)(tile_nz[tile + 1] - y0);  // one past its last
   const Off origin = y0 - lead;           // nonzero at place 0, a multiple of E
   const int q = E * tid;                  // this thread's first place
 
@@ -210,7 +208,7 @@ mp_spmv_kernel(const Off* __restrict__ row_end, const int32_t* __restrict__ col,
 #pragma unroll
     for (int j = 0; j < E; ++j) {
       const bool in = q + j >= lead && q + j < end;
-      xv[j] = in ? __ldg(x + c[j]) : V(0);
+      xv[j] = in ? ld_prev(x + c[j]) : V(0);
       if (!in) v[j] = V(0);
     }
   }
@@ -279,12 +277,12 @@ mp_spmv_kernel(const Off* __restrict__ row_end, const int32_t* __restrict__ col,
       }
       if (first != kNoRow) y[x0 + first] = s;
       if (last) {
-        carry_row[tile] = x1;
+        carry_row[tile] = x0 + nrows;
         carry_val[tile] = first != kNoRow ? acc : s;
       }
     }
     if (tid == 0 && end == lead) {
-      carry_row[tile] = x1;
+      carry_row[tile] = x0 + nrows;
       carry_val[tile] = V(0);
     }
     return;
@@ -311,7 +309,7 @@ mp_spmv_kernel(const Off* __restrict__ row_end, const int32_t* __restrict__ col,
     }
     sum = rake_scan(sum, ends, lane);
     if (lane == 31) {
-      carry_row[tile] = x1;
+      carry_row[tile] = x0 + nrows;
       carry_val[tile] = sum;
     }
     sum = __shfl_up_sync(kFull, sum, 1);
@@ -337,7 +335,7 @@ mp_spmv_kernel(const Off* __restrict__ row_end, const int32_t* __restrict__ col,
   }
   sum = rake_scan(sum, ends, lane);
   if (lane == 31) {
-    carry_row[tile] = x1;
+    carry_row[tile] = x0 + nrows;
     carry_val[tile] = sum;
   }
   sum = __shfl_up_sync(kFull, sum, 1);
@@ -359,8 +357,7 @@ mp_spmv_kernel(const Off* __restrict__ row_end, const int32_t* __restrict__ col,
 // warp, lane l taking tiles l, l + 32, ... of the run, joined by a fixed xor
 // tree, so a hub row costs a few loads in a row instead of one per tile.
 template <typename V, typename Off>
-__global__ void mp_fixup_kernel(const Off* __restrict__ carry_row, const V* __restrict__ carry_val,
-                                long long num_tiles, Off n_rows, V* __restrict__ y) {
+__global__ void mp_fixup_kernel(const Off* carry_row, const V* carry_val, long long num_tiles, Off n_rows, V* y) {
   constexpr unsigned kFull = 0xffffffffu;
   constexpr int kShort = 4;
   release_next();

@@ -7,8 +7,8 @@
 // (VW = 1: the reference's cross-row kernel, one lane per row, no reduction).
 // CHUNK tasks do the same for 32-wide pieces of long rows and a second launch
 // adds the pieces of each long row in chunk order.  Values and columns are
-// read once (no L1 allocation, L2 evict-first policy); x is gathered through
-// the read-only path with evict-last policies.
+// read once (no L1 allocation, L2 evict-first policy); x is gathered by
+// ordinary loads (launch.cuh).
 // FP64 work: one FMA per entry plus log2(VW) adds per row.
 
 #include <cuda_runtime.h>
@@ -58,12 +58,12 @@ __device__ __forceinline__ int ld_once(const int* p, unsigned long long pol) {
 }
 __device__ __forceinline__ double ld_keep(const double* p, unsigned long long pol) {
   double v;
-  asm("ld.global.nc.L1::evict_last.L2::cache_hint.f64 %0, [%1], %2;" : "=d"(v) : "l"(p), "l"(pol));
+  asm volatile("ld.global.L1::evict_last.L2::cache_hint.f64 %0, [%1], %2;" : "=d"(v) : "l"(p), "l"(pol));
   return v;
 }
 __device__ __forceinline__ float ld_keep(const float* p, unsigned long long pol) {
   float v;
-  asm("ld.global.nc.L1::evict_last.L2::cache_hint.f32 %0, [%1], %2;" : "=f"(v) : "l"(p), "l"(pol));
+  asm volatile("ld.global.L1::evict_last.L2::cache_hint.f32 %0, [%1], %2;" : "=f"(v) : "l"(p), "l"(pol));
   return v;
 }
 
@@ -85,17 +85,17 @@ __device__ __forceinline__ int ld_na(const int* p) {
 }
 __device__ __forceinline__ double ld_l1_keep(const double* p) {
   double v;
-  asm("ld.global.nc.L1::evict_last.f64 %0, [%1];" : "=d"(v) : "l"(p));
+  asm volatile("ld.global.L1::evict_last.f64 %0, [%1];" : "=d"(v) : "l"(p));
   return v;
 }
 __device__ __forceinline__ float ld_l1_keep(const float* p) {
   float v;
-  asm("ld.global.nc.L1::evict_last.f32 %0, [%1];" : "=f"(v) : "l"(p));
+  asm volatile("ld.global.L1::evict_last.f32 %0, [%1];" : "=f"(v) : "l"(p));
   return v;
 }
 
 // Cache-hint variants H: 0 streaming (.cs) loads of values/columns and
-// read-only x gathers; 1 explicit L1/L2 policies; 2 values/columns without L1
+// plain x gathers; 1 explicit L1/L2 policies; 2 values/columns without L1
 // allocation; 3 as 2 with x gathers marked L1 evict-last.
 template <int H, typename T> __device__ __forceinline__ T ld_stream_h(const T* p, const Policies& pol) {
   if constexpr (H == 0) return __ldcs(p);
@@ -103,7 +103,7 @@ template <int H, typename T> __device__ __forceinline__ T ld_stream_h(const T* p
   else return ld_na(p);
 }
 template <int H, typename T> __device__ __forceinline__ T ld_x_h(const T* p, const Policies& pol) {
-  if constexpr (H == 0 || H == 2) return __ldg(p);
+  if constexpr (H == 0 || H == 2) return ld_prev(p);
   else if constexpr (H == 1) return ld_keep(p, pol.keep);
   else return ld_l1_keep(p);
 }
@@ -148,8 +148,7 @@ constexpr int kDenseShort = 10;
 template <typename V, int U>
 __global__ void __launch_bounds__(kWarpsPerBlock * 32)
 dense_block_kernel(const SlicedTask* __restrict__ tasks, long long num_tasks, const V* __restrict__ val,
-                   const int32_t* __restrict__ col, const int32_t* __restrict__ rowid, const V* __restrict__ x,
-                   int n_cols, V* __restrict__ y, V* __restrict__ chunk_sum) {
+                   const int32_t* __restrict__ col, const int32_t* __restrict__ rowid, const V* x, int n_cols, V* y, V* chunk_sum) {
   const long long w = ((long long)blockIdx.x * kWarpsPerBlock) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   release_next();
@@ -179,7 +178,7 @@ dense_block_kernel(const SlicedTask* __restrict__ tasks, long long num_tasks, co
       if (k + u < steps) {
         V xv[4];
 #pragma unroll
-        for (int l = 0; l < 4; ++l) xv[l] = c[u] + l < n_cols ? __ldg(x + c[u] + l) : V(0);
+        for (int l = 0; l < 4; ++l) xv[l] = c[u] + l < n_cols ? ld_prev(x + c[u] + l) : V(0);
 #pragma unroll
         for (int l = 0; l < 4; ++l) acc = fmav<V>(v[u][l], xv[l], acc);
       }
@@ -195,7 +194,7 @@ dense_block_kernel(const SlicedTask* __restrict__ tasks, long long num_tasks, co
 
 // Address of x for a (possibly hot-relabelled) column.
 template <bool HOT, typename V>
-__device__ __forceinline__ const V* x_at(const V* __restrict__ x, const V* __restrict__ xh, int ncols, int c) {
+__device__ __forceinline__ const V* x_at(const V* x, const V* xh, int ncols, int c) {
   if constexpr (HOT) return c < ncols ? x + c : xh + (c - ncols);
   else return x + c;
 }
@@ -221,8 +220,8 @@ __device__ __forceinline__ V epi_out(V acc, int row, const SlicedEpilogue& ep) {
 template <typename V, int U, int H, bool HOT, bool EPI, bool SH = false>
 __device__ __forceinline__ void sliced_task(long long w, int lane, const SlicedTask* __restrict__ tasks,
                                             const V* __restrict__ val, const int32_t* __restrict__ col,
-                                            const int32_t* __restrict__ rowid, const V* __restrict__ x, V* y,
-                                            V* __restrict__ chunk_sum, const V* __restrict__ xh, int ncols,
+                                            const int32_t* __restrict__ rowid, const V* x, V* y, V* chunk_sum,
+                                            const V* xh, int ncols,
                                             const SlicedEpilogue& ep, const uint16_t* __restrict__ col16,
                                             const int32_t* __restrict__ first,
                                             const SlicedPrefetch& pf = SlicedPrefetch(),
@@ -265,7 +264,7 @@ __device__ __forceinline__ void sliced_task(long long w, int lane, const SlicedT
       for (int u = 0; u < U; ++u) v[u] = __ldcs(vp + (k + u) * 32);
       pattern_at<U>(offs, k, o);
 #pragma unroll
-      for (int u = 0; u < U; ++u) xv[u] = __ldg(xr + o[u]);
+      for (int u = 0; u < U; ++u) xv[u] = ld_prev(xr + o[u]);
 #pragma unroll
       for (int u = 0; u < U; ++u) acc = fmav<V>(v[u], xv[u], acc);
     }
@@ -278,7 +277,7 @@ __device__ __forceinline__ void sliced_task(long long w, int lane, const SlicedT
       pattern_at<4>(offs, k, o);
 #pragma unroll
       for (int u = 0; u < 4; ++u)
-        if (k + u < steps) xv[u] = __ldg(xr + o[u]);
+        if (k + u < steps) xv[u] = ld_prev(xr + o[u]);
 #pragma unroll
       for (int u = 0; u < 4; ++u)
         if (k + u < steps) acc = fmav<V>(v[u], xv[u], acc);
@@ -310,13 +309,13 @@ __device__ __forceinline__ void sliced_task(long long w, int lane, const SlicedT
         cc[u] = c;
       }
 #pragma unroll
-      for (int u = 0; u < U; ++u) xv[u] = __ldg(x_at<HOT>(x, xh, ncols, cc[u]));
+      for (int u = 0; u < U; ++u) xv[u] = ld_prev(x_at<HOT>(x, xh, ncols, cc[u]));
 #pragma unroll
       for (int u = 0; u < U; ++u) acc = fmav<V>(v[u], xv[u], acc);
     }
     for (; k < steps; ++k) {
       c += __ldcs(dp + k * 32);
-      acc = fmav<V>(__ldcs(vp + k * 32), __ldg(x_at<HOT>(x, xh, ncols, c)), acc);
+      acc = fmav<V>(__ldcs(vp + k * 32), ld_prev(x_at<HOT>(x, xh, ncols, c)), acc);
     }
     if (lane < nrows) {
       const int row = rowid[row_base + lane];
@@ -361,8 +360,8 @@ __device__ __forceinline__ void sliced_task(long long w, int lane, const SlicedT
 template <typename V, int U, int H, bool HOT = false, bool EPI = false, bool SH = false>
 __global__ void __launch_bounds__(kWarpsPerBlock * 32)
 sliced_kernel(const SlicedTask* __restrict__ tasks, long long num_tasks, const V* __restrict__ val,
-              const int32_t* __restrict__ col, const int32_t* __restrict__ rowid, const V* __restrict__ x,
-              V* y, V* __restrict__ chunk_sum, const V* __restrict__ xh = nullptr, int ncols = 0,
+              const int32_t* __restrict__ col, const int32_t* __restrict__ rowid, const V* x, V* y, V* chunk_sum,
+              const V* xh = nullptr, int ncols = 0,
               SlicedEpilogue ep = SlicedEpilogue(), const uint16_t* __restrict__ col16 = nullptr,
               const int32_t* __restrict__ first = nullptr, SlicedPrefetch pf = SlicedPrefetch(),
               const uint16_t* __restrict__ pat16 = nullptr) {
@@ -382,8 +381,8 @@ template <bool HOT>
 __global__ void __launch_bounds__(kWarpsPerBlock * 32)
 sliced_guard_kernel(int* guard, const SlicedTask* __restrict__ tasks, long long num_tasks,
                     const double* __restrict__ val, const int32_t* __restrict__ col,
-                    const int32_t* __restrict__ rowid, const double* __restrict__ x, double* y,
-                    double* __restrict__ chunk_sum, const double* __restrict__ xh, int ncols,
+                    const int32_t* __restrict__ rowid, const double* x, double* y, double* chunk_sum,
+                    const double* xh, int ncols,
                     const uint16_t* __restrict__ col16, const int32_t* __restrict__ first) {
   release_next();
   wait_for_previous();
@@ -403,7 +402,7 @@ sliced_guard_kernel(int* guard, const SlicedTask* __restrict__ tasks, long long 
 template <typename V, bool EPI = false>
 __global__ void sliced_long_fixup(const int32_t* __restrict__ long_row, const int32_t* __restrict__ long_first,
                                   const int32_t* __restrict__ long_heavy, long long num_long, long long num_heavy,
-                                  long long heavy_sub, unsigned light_blocks, const V* __restrict__ chunk_sum, V* y,
+                                  long long heavy_sub, unsigned light_blocks, const V* chunk_sum, V* y,
                                   SlicedEpilogue ep = SlicedEpilogue()) {
   release_next();
   wait_for_previous();
@@ -440,12 +439,12 @@ bool launch_dense(const SlicedMatrix& m, const void* x, void* y, cudaStream_t s)
 }
 
 template <typename V>
-__global__ void gather_hot(const V* __restrict__ x, const int32_t* __restrict__ hot_cols, int n, V* __restrict__ xh) {
+__global__ void gather_hot(const V* x, const int32_t* __restrict__ hot_cols, int n, V* xh) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   release_next();
   const int c = i < n ? __ldg(hot_cols + i) : 0;
   wait_for_previous();
-  if (i < n) xh[i] = __ldg(x + c);
+  if (i < n) xh[i] = ld_prev(x + c);
 }
 
 template <typename V>

@@ -108,7 +108,7 @@ namespace {
 
 // x (n values) followed by the values of the `nh` hot columns (a plan with a
 // hot-column window reads slot s as column n + s).
-__device__ __forceinline__ double x_ext(const double* __restrict__ x, long long n, const int32_t* __restrict__ hot,
+__device__ __forceinline__ double x_ext(const double* x, long long n, const int32_t* __restrict__ hot,
                                         long long i) {
   return x[i < n ? i : __ldg(hot + (i - n))];
 }
@@ -119,15 +119,15 @@ __device__ __forceinline__ bool aligned16(const void* p) { return (reinterpret_c
 // consecutive values per step (two 16-byte loads, one 16-byte store) when x is
 // 16-byte aligned, so enough bytes are in flight to run at HBM rate; the
 // remainder and the hot tail take one value per step.
-__device__ __forceinline__ void round_x(const double* __restrict__ x, float* __restrict__ x32, long long n,
-                                        const int32_t* __restrict__ hot, int nh) {
+__device__ __forceinline__ void round_x(const double* x, float* x32, long long n, const int32_t* __restrict__ hot,
+                                        int nh) {
   const long long t0 = blockIdx.x * (long long)blockDim.x + threadIdx.x, nt = (long long)gridDim.x * blockDim.x;
   release_next();
   wait_for_previous();
   const long long n4 = aligned16(x) && aligned16(x32) ? n / 4 : 0;
   for (long long q = t0; q < n4; q += nt) {
-    const double2 a = __ldcs(reinterpret_cast<const double2*>(x) + 2 * q);
-    const double2 b = __ldcs(reinterpret_cast<const double2*>(x) + 2 * q + 1);
+    const double2 a = ld_prev_once(reinterpret_cast<const double2*>(x) + 2 * q);
+    const double2 b = ld_prev_once(reinterpret_cast<const double2*>(x) + 2 * q + 1);
     reinterpret_cast<float4*>(x32)[q] =
         make_float4(f64_to_f32_rne(a.x), f64_to_f32_rne(a.y), f64_to_f32_rne(b.x), f64_to_f32_rne(b.y));
   }
@@ -137,19 +137,19 @@ __device__ __forceinline__ void round_x(const double* __restrict__ x, float* __r
 }  // namespace
 
 // Outside the anonymous namespace: also launched by SpB_VNEC_f64_to_f32_ext.
-__global__ void x_to_f32_kernel(const double* __restrict__ x, float* __restrict__ x32, long long n) {
+__global__ void x_to_f32_kernel(const double* x, float* x32, long long n) {
   round_x(x, x32, n, nullptr, 0);
 }
 namespace {
 
-__global__ void x_to_f32_ext_kernel(const double* __restrict__ x, float* __restrict__ x32, long long n,
-                                    const int32_t* __restrict__ hot, int nh) {
+__global__ void x_to_f32_ext_kernel(const double* x, float* x32, long long n, const int32_t* __restrict__ hot,
+                                    int nh) {
   round_x(x, x32, n, hot, nh);
 }
 
 // x split into (hi, lo) pairs, then the hot columns' pairs: two values per
 // step (one 16-byte load, one 16-byte store) when x is 16-byte aligned.
-__global__ void x_split_kernel(const double* __restrict__ x, float2* __restrict__ xs, long long n, int* flag,
+__global__ void x_split_kernel(const double* x, float2* xs, long long n, int* flag,
                                const int32_t* __restrict__ hot, int nh) {
   const long long t0 = blockIdx.x * (long long)blockDim.x + threadIdx.x, nt = (long long)gridDim.x * blockDim.x;
   release_next();
@@ -157,7 +157,7 @@ __global__ void x_split_kernel(const double* __restrict__ x, float2* __restrict_
   const long long n2 = aligned16(x) && aligned16(xs) ? n / 2 : 0;
   bool bad = false;
   for (long long q = t0; q < n2; q += nt) {
-    const double2 a = __ldcs(reinterpret_cast<const double2*>(x) + q);
+    const double2 a = ld_prev_once(reinterpret_cast<const double2*>(x) + q);
     float h0, l0, h1, l1;
     bad |= !df_split(a.x, h0, l0);
     bad |= !df_split(a.y, h1, l1);
@@ -178,7 +178,7 @@ struct CodecF32 {
   __device__ static const void* at(const void* xs, int c) { return static_cast<const float*>(xs) + c; }
   __device__ static Acc zero() { return 0.0f; }
   __device__ static Acc mac(Acc a, Val v, const void* xs, int c) {
-    return fmaf(v, __ldg(static_cast<const float*>(xs) + c), a);
+    return fmaf(v, ld_prev(static_cast<const float*>(xs) + c), a);
   }
   __device__ static double to_f64(Acc a) { return widen(a); }
 };
@@ -190,7 +190,8 @@ struct CodecBF16 {
   __device__ static const void* at(const void* xs, int c) { return static_cast<const float*>(xs) + c; }
   __device__ static Acc zero() { return 0.0f; }
   __device__ static Acc mac(Acc a, Val v, const void* xs, int c) {
-    return fmaf(__uint_as_float(static_cast<unsigned>(v) << 16), __ldg(static_cast<const float*>(xs) + c), a);
+    // A plain dereference: behind the wait too, and 32 registers in place of 40 at 12 steps (stencil 100^3 24.1, not 26.5 us).
+    return fmaf(__uint_as_float(static_cast<unsigned>(v) << 16), static_cast<const float*>(xs)[c], a);
   }
   __device__ static double to_f64(Acc a) { return widen(a); }
 };
@@ -202,7 +203,7 @@ struct CodecDF32 {
   __device__ static const void* at(const void* xs, int c) { return static_cast<const float2*>(xs) + c; }
   __device__ static Acc zero() { return DF{0.0f, 0.0f}; }
   __device__ static Acc mac(Acc acc, Val v, const void* xs, int c) {
-    const float2 x = __ldg(static_cast<const float2*>(xs) + c);
+    const float2 x = ld_prev(static_cast<const float2*>(xs) + c);
     return df_mac(acc, v.x, v.y, x.x, x.y);
   }
   __device__ static double to_f64(Acc a) { return df_to_f64(a); }
@@ -215,7 +216,7 @@ struct CodecF32Direct : CodecF32 {
   static constexpr bool kDirect = true;
   __device__ static const void* at(const void* xs, int c) { return static_cast<const double*>(xs) + c; }
   __device__ static Acc mac(Acc a, Val v, const void* xs, int c) {
-    return fmaf(v, __double2float_rn(__ldg(static_cast<const double*>(xs) + c)), a);
+    return fmaf(v, __double2float_rn(ld_prev(static_cast<const double*>(xs) + c)), a);
   }
 };
 struct CodecBF16Direct : CodecBF16 {
@@ -223,7 +224,7 @@ struct CodecBF16Direct : CodecBF16 {
   __device__ static const void* at(const void* xs, int c) { return static_cast<const double*>(xs) + c; }
   __device__ static Acc mac(Acc a, Val v, const void* xs, int c) {
     return fmaf(__uint_as_float(static_cast<unsigned>(v) << 16),
-                __double2float_rn(__ldg(static_cast<const double*>(xs) + c)), a);
+                __double2float_rn(ld_prev(static_cast<const double*>(xs) + c)), a);
   }
 };
 struct CodecDF32Direct : CodecDF32 {
@@ -236,7 +237,7 @@ struct CodecDF32Direct : CodecDF32 {
   __device__ static Acc zero() { return Acc{DF{0.0f, 0.0f}, false}; }
   __device__ static Acc mac(Acc a, Val v, const void* xs, int c) {
     float h, l;
-    const bool ok = df_split(__ldg(static_cast<const double*>(xs) + c), h, l);
+    const bool ok = df_split(ld_prev(static_cast<const double*>(xs) + c), h, l);
     return Acc{df_mac(a.sum, v.x, v.y, h, l), a.bad || !ok};
   }
   __device__ static double to_f64(const Acc& a) { return df_to_f64(a.sum); }
@@ -299,14 +300,19 @@ __device__ __forceinline__ double scale2(double s, int e) {
 // in the same order as the stride-32 layout (P = 0), so both give the same y.
 // SH: the plan has shared-pattern tasks (kSlicedShared); plans without them
 // run the SH = false build, whose registers the shared path does not raise.
+// Six blocks an SM (40 registers) for the shared-pattern builds that take 42 to 48
+// left alone.
 template <class C, int U, int P, bool SH>
-__global__ void __launch_bounds__(kWarps * 32)
+constexpr int kMixedBlocks = SH && ((std::is_same<C, CodecBF16>::value && P > 0 && U != 12) ||
+                                    (std::is_same<C, CodecDF32>::value && U == 16)) ? 6 : 0;
+
+template <class C, int U, int P, bool SH>
+__global__ void __launch_bounds__(kWarps * 32, kMixedBlocks<C, U, P, SH>)
 sliced_mixed_kernel(const SlicedTask* __restrict__ tasks, long long num_tasks, const typename C::Val* __restrict__ val,
-                    const int32_t* __restrict__ col, const int32_t* __restrict__ rowid, const void* __restrict__ xs,
-                    double* __restrict__ y, double* __restrict__ chunk_sum, const signed char* __restrict__ row_scale,
-                    const signed char* __restrict__ chunk_scale, int* flag,
-                    const uint16_t* __restrict__ col16, const int32_t* __restrict__ first,
-                    const uint16_t* __restrict__ pat16, SlicedPrefetch pf) {
+                    const int32_t* __restrict__ col, const int32_t* __restrict__ rowid, const void* xs, double* y,
+                    double* chunk_sum, const signed char* __restrict__ row_scale,
+                    const signed char* __restrict__ chunk_scale, int* flag, const uint16_t* __restrict__ col16,
+                    const int32_t* __restrict__ first, const uint16_t* __restrict__ pat16, SlicedPrefetch pf) {
   const long long w = ((long long)blockIdx.x * kWarps) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   release_next();
@@ -616,8 +622,7 @@ sliced_mixed_kernel(const SlicedTask* __restrict__ tasks, long long num_tasks, c
 
 __global__ void long_fixup_f64(const int32_t* __restrict__ long_row, const int32_t* __restrict__ long_first,
                                const int32_t* __restrict__ long_heavy, long long num_long, long long num_heavy,
-                               long long heavy_sub, unsigned light_blocks, const double* __restrict__ chunk_sum,
-                               double* __restrict__ y) {
+                               long long heavy_sub, unsigned light_blocks, const double* chunk_sum, double* y) {
   release_next();
   wait_for_previous();
   long_rows_fixup<double>(long_first, long_heavy, num_long, num_heavy, heavy_sub, light_blocks, chunk_sum,

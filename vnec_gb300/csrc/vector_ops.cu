@@ -43,8 +43,7 @@ constexpr long long kDotBlockValues = (long long)kDotTpb * 2 * kDotPairs;
 // 16-byte aligned.
 template <int MODE>
 __global__ void __launch_bounds__(kDotTpb)
-dot_partial_kernel(long long n, const double* __restrict__ a, const double* __restrict__ b, bool vec,
-                   double* __restrict__ partial) {
+dot_partial_kernel(long long n, const double* a, const double* b, bool vec, double* partial) {
   __shared__ double sh[kDotTpb / 32];
   release_next();
   wait_for_previous();
@@ -63,24 +62,24 @@ dot_partial_kernel(long long n, const double* __restrict__ a, const double* __re
     double2 u[kDotPairs], v[kDotPairs];
 #pragma unroll
     for (int j = 0; j < kDotPairs; ++j) {
-      u[j] = __ldg(a2 + q + j * stride);
-      v[j] = __ldg(b2 + q + j * stride);
+      u[j] = ld_prev(a2 + q + j * stride);
+      v[j] = ld_prev(b2 + q + j * stride);
     }
 #pragma unroll
     for (int j = 0; j < kDotPairs; ++j) acc[j] = add(add(acc[j], u[j].x, v[j].x), u[j].y, v[j].y);
   }
   for (; q < n2; q += stride) {
-    const double2 u = __ldg(a2 + q), v = __ldg(b2 + q);
+    const double2 u = ld_prev(a2 + q), v = ld_prev(b2 + q);
     acc[0] = add(add(acc[0], u.x, v.x), u.y, v.y);
   }
 #pragma unroll 4
-  for (long long i = 2 * n2 + t; i < n; i += stride) acc[0] = add(acc[0], __ldg(a + i), __ldg(b + i));
+  for (long long i = 2 * n2 + t; i < n; i += stride) acc[0] = add(acc[0], ld_prev(a + i), ld_prev(b + i));
   const double s = block_sum((acc[0] + acc[1]) + (acc[2] + acc[3]), sh);
   if (threadIdx.x == 0) partial[blockIdx.x] = s;
 }
 
 __global__ void __launch_bounds__(kDotTpb)
-dot_final_kernel(const double* __restrict__ partial, int n, double* __restrict__ out) {
+dot_final_kernel(const double* partial, int n, double* out) {
   __shared__ double sh[kDotTpb / 32];
   release_next();
   wait_for_previous();
