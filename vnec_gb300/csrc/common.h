@@ -95,10 +95,13 @@ struct DeviceBuffer {
   template <typename T> T* as() const { return static_cast<T*>(ptr); }
 };
 
-// Owning page-locked host allocation that kernels write to (`dev`).
+// Owning page-locked host allocation that kernels write to (`dev`).  Where there
+// is none to be had, alloc() returns false, keeps nothing and sets no error: its
+// callers go another way.
 struct MappedBuffer {
   void* host = nullptr;
   void* dev = nullptr;
+  bool refused = false;  // asked for once already, in vain
   MappedBuffer() = default;
   MappedBuffer(const MappedBuffer&) = delete;
   MappedBuffer& operator=(const MappedBuffer&) = delete;
@@ -106,11 +109,17 @@ struct MappedBuffer {
     if (host) cudaFreeHost(host);
   }
   bool alloc(size_t n) {
-    if (!VNEC_CUDA(cudaHostAlloc(&host, n, cudaHostAllocMapped | cudaHostAllocPortable))) {
-      host = nullptr;
-      return false;
+    void *h = nullptr, *d = nullptr;
+    const bool got = cudaHostAlloc(&h, n, cudaHostAllocMapped | cudaHostAllocPortable) == cudaSuccess;
+    if (got && cudaHostGetDevicePointer(&d, h, 0) == cudaSuccess) {
+      host = h;
+      dev = d;
+      return true;
     }
-    return VNEC_CUDA(cudaHostGetDevicePointer(&dev, host, 0));
+    cudaGetLastError();
+    if (got) cudaFreeHost(h);
+    refused = true;
+    return false;
   }
 };
 

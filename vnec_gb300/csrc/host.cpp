@@ -261,10 +261,9 @@ bool Plan::run_host(const void* h_x, void* h_y) {
   // whatever it moves (3,001 values: call 25.5 -> 14 us; 8,192: 27 -> 18; from
   // 32,768 on the two are equal, and longer the CPU's copy loses: 131,072 values
   // 45 us by copy engine, 130 by CPU).  Not for push plans, whose atomics would
-  // go over the link.
+  // go over the link, nor where no page-locked memory is to be had.
   constexpr size_t kDirectBytes = 128 << 10;
-  if (ny > 0 && vb * ny <= kDirectBytes && kind != PlanKind::kPush) {
-    if (!hy.host && !hy.alloc(vb * ny)) return false;
+  if (ny > 0 && vb * ny <= kDirectBytes && kind != PlanKind::kPush && (hy.host || (!hy.refused && hy.alloc(vb * ny)))) {
     if (nx > 0 && !VNEC_CUDA(cudaMemcpyAsync(dx.ptr, h_x, vb * nx, cudaMemcpyHostToDevice, own_stream))) return false;
     if (!run(dx.ptr, hy.dev, own_stream)) return false;
     const bool ok = device_status(own_stream);
