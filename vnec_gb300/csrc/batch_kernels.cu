@@ -121,7 +121,7 @@ template <bool VEC, int R> __device__ __forceinline__ void store_y(double* p, co
 }
 
 struct CodecF64 {
-  static constexpr bool kPairReduce = false, kOwnX = false, kAhead = false;
+  static constexpr bool kPairReduce = false, kOwnX = false;
   using V = double;
   using X = double;
   struct A {
@@ -133,7 +133,7 @@ struct CodecF64 {
 };
 
 struct CodecF32 {
-  static constexpr bool kPairReduce = false, kOwnX = true, kAhead = true;
+  static constexpr bool kPairReduce = false, kOwnX = true;
   using V = float;
   using X = float;
   struct A {
@@ -147,7 +147,7 @@ struct CodecF32 {
 // Double-float: value (hi, lo) times x (hi, lo), Dekker product with FMA,
 // TwoSum into (s, c).
 struct CodecDF32 {
-  static constexpr bool kPairReduce = true, kOwnX = true, kAhead = true;
+  static constexpr bool kPairReduce = true, kOwnX = true;
   using V = float2;
   using X = float2;
   struct A {
@@ -183,7 +183,7 @@ struct CodecDF32 {
 
 // FP64 from split values and FP64 X: the guard path of DF32 plans.
 struct CodecDF32Guard {
-  static constexpr bool kPairReduce = false, kOwnX = false, kAhead = false;
+  static constexpr bool kPairReduce = false, kOwnX = false;
   using V = float2;
   using X = double;
   struct A {
@@ -214,9 +214,9 @@ constexpr int kStageRounds = 4;
 // A layout of L lanes per slot then runs with L >> TL lanes that hold 2^TL times
 // the right-hand sides: every slot's sums are those of TL = 0, bit for bit, but
 // fewer lanes read each column and value and X comes in wider loads.
-template <class Cd, int R, int U, bool STAGED, bool VEC, int TL = 0>
+template <class Cd, int R, int U, bool STAGED, bool VEC, bool AHEAD, bool HALVE, int TL = 0>
 __device__ __forceinline__ void run_tasks(const BatchArgs& a, const typename Cd::X* x) {
-  static_assert(TL == 0 || (!STAGED && Cd::kAhead), "several tasks per warp run the fetch-ahead loop");
+  static_assert(TL == 0 || (!STAGED && AHEAD), "several tasks per warp run the fetch-ahead loop");
   using V = typename Cd::V;
   using X = typename Cd::X;
   constexpr int W = 32 >> TL;  // lanes of a task
@@ -287,7 +287,7 @@ __device__ __forceinline__ void run_tasks(const BatchArgs& a, const typename Cd:
       }
       s = steps;
     }
-    if constexpr (Cd::kAhead) {
+    if constexpr (AHEAD) {
       // U steps at a time; the next U steps' columns and values are fetched before
       // these steps' X rows are waited for.
       if (s < steps) {
@@ -355,7 +355,14 @@ __device__ __forceinline__ void run_tasks(const BatchArgs& a, const typename Cd:
     double d[R];
     int width = R, at = 0;  // this lane ends with right-hand sides [at, at + width) of its R
     bool writes = true;
-    if constexpr (Cd::kPairReduce) {
+    if constexpr (!HALVE) {
+#pragma unroll
+      for (int r = 0; r < R; ++r) d[r] = Cd::out(acc[r]);
+      for (int off = 1 << ll; off < span; off <<= 1)
+#pragma unroll
+        for (int r = 0; r < R; ++r) d[r] += __shfl_xor_sync(kFull, d[r], off);
+      writes = kind == kSlicedChunk ? slot == 0 : (slot & ((1 << vwl) - 1)) == 0;
+    } else if constexpr (Cd::kPairReduce) {
       // Double-float: sum the slots as (hi, lo) pairs on the FP32 pipe and
       // convert once (each FP64 operation costs 64 FP32 issue slots here).
 #pragma unroll
@@ -437,35 +444,66 @@ __device__ __forceinline__ void run_tasks(const BatchArgs& a, const typename Cd:
   }
 }
 
-template <class Cd, int R, int U, bool STAGED, bool VEC, int TL = 0>
-__global__ void __launch_bounds__(256) batch_kernel(const BatchArgs a) {
+template <class Cd, int R, int U, bool STAGED, bool VEC, bool AHEAD, bool HALVE, int TL, int B>
+__global__ void __launch_bounds__(256, B) batch_kernel(const BatchArgs a) {
   release_next();
   wait_for_previous();
-  run_tasks<Cd, R, U, STAGED, VEC, TL>(a, static_cast<const typename Cd::X*>(a.x));
+  run_tasks<Cd, R, U, STAGED, VEC, AHEAD, HALVE, TL>(a, static_cast<const typename Cd::X*>(a.x));
 }
 
-template <int R, int U, bool STAGED, bool VEC>
+// UG: the guard's steps in flight; its loop neither stages nor fetches ahead, so
+// that it does not raise the kernel's registers.
+template <int R, int U, int UG, bool STAGED, bool VEC, bool AHEAD>
 __global__ void __launch_bounds__(256) batch_df32_kernel(const BatchArgs a) {
   release_next();
   wait_for_previous();
   if (*reinterpret_cast<const volatile int*>(a.flag))
-    run_tasks<CodecDF32Guard, R, U, STAGED, VEC>(a, a.x64);
+    run_tasks<CodecDF32Guard, R, UG, false, VEC, false, true>(a, a.x64);
   else
-    run_tasks<CodecDF32, R, U, STAGED, VEC>(a, static_cast<const float2*>(a.x));
+    run_tasks<CodecDF32, R, U, STAGED, VEC, AHEAD, true>(a, static_cast<const float2*>(a.x));
 }
 
-// Steps in flight per lane: 8 / R (at least 2), doubled in mode 1; mode 2
-// stages the entries in registers (STAGED) with the mode-0 step count.
-template <int R, int MODE> constexpr int unroll_for() { return (R >= 4 ? 2 : 8 / R) * (MODE == 1 ? 2 : 1); }
+// Steps in flight per lane: 8 / R (at least 2), doubled in mode 1; mode 2 stages
+// the entries in registers with the mode-0 step count.  The fetch-ahead loops (modes
+// 0 and 1 of FP32 and DF32) hold the next steps' columns and values too, and the
+// double-float pairs are twice as wide, so there the full count costs more warps
+// than it hides: 112 to 238 registers where these take 64 to 128.  Explicit layouts
+// of 14 M nonzeros and, in brackets, 0.8 M, time against the loop without
+// fetch-ahead at mode 1's full count (geometric means over k and chunk lengths):
+//   DF32   R = 1: 16 steps 1.74 (0.63), 8 0.96 (0.46), 6 0.74 (0.43), 5 0.66 (0.44), 4 0.68 (0.44);
+//          staged 8 against 4: 1.78 (1.80)
+//          R = 2:  8 steps 0.97 (0.47), 6 0.95 (0.45), 4 0.79 (0.45), 3 0.71 (0.45)
+//          R = 4:  4 steps 0.89 (0.48), 3 0.77 (0.49), 2 0.76 (0.53)
+//          R = 8:  4 steps 1.10 (0.48), 3 0.79 (0.46), 2 0.83 (0.46)
+//   FP32   R = 1: 16 steps 1.15 (0.59), 12 1.08 (0.58), 8 0.96 (0.72), 6 0.80 (0.62), 4 0.81 (0.76)
+//          R = 2:  8 steps 1.06 (0.81), 6 0.82 (0.68), 5 0.84 (0.71), 4 0.85 (0.69)
+//          R = 4:  4 steps 0.77 (0.62), 3 0.73 (0.57), 2 0.79 (0.63)
+//          R = 8:  4 steps 0.78 (0.48), 3 0.69 (0.54), 2 0.68 (0.58)
+constexpr int steps_in_flight(int precision, int R, int mode) {
+  if (precision == kPrecDF32) {
+    if (R == 1) return mode == 1 ? 5 : 4;
+    if (mode == 1 || (mode == 0 && R != 4)) return 3;
+  }
+  if (precision == kPrecFP32) {
+    if (mode == 1 && R == 4) return 3;
+    if ((mode == 1 && R <= 2) || (mode == 0 && R == 1)) return 6;
+  }
+  return (R >= 4 ? 2 : 8 / R) * (mode == 1 ? 2 : 1);
+}
 
 using BatchKernel = void (*)(BatchArgs);
 template <int R, int MODE, bool VEC> BatchKernel kernel_for(int precision) {
-  constexpr int U = unroll_for<R, MODE>();
-  constexpr bool ST = MODE == 2;
+  constexpr bool ST = MODE == 2, AHEAD = !ST;
   switch (precision) {
-    case kPrecFP32: return &batch_kernel<CodecF32, R, U, ST, VEC>;
-    case kPrecDF32: return &batch_df32_kernel<R, U, ST, VEC>;
-    default: return &batch_kernel<CodecF64, R, U, ST, VEC>;
+    case kPrecFP32:
+      return &batch_kernel<CodecF32, R, steps_in_flight(kPrecFP32, R, MODE), ST, VEC, AHEAD, true, 0,
+                           ST && R == 1 ? 4 : 0>;  // 64 registers, not 80: 14 M nonzeros 1.13x, 0.8 M 1.01x
+    case kPrecDF32:
+      return &batch_df32_kernel<R, steps_in_flight(kPrecDF32, R, MODE), steps_in_flight(kPrecFP64, R, 0), ST, VEC, AHEAD>;
+    default:
+      // R of 1 and 2 with twice the steps: the plain butterfly leaves the compiler
+      // a better schedule (1.06 to 1.5x over k and sizes; R = 4, 8: 0.9x).
+      return &batch_kernel<CodecF64, R, steps_in_flight(kPrecFP64, R, MODE), ST, VEC, false, !(MODE == 1 && R <= 2), 0, 0>;
   }
 }
 
@@ -478,13 +516,13 @@ template <int R, bool VEC = true> BatchKernel kernel_for_mode(int precision, int
 // Several FP32 tasks per warp (BatchMatrix::tasks_log2), by the right-hand sides
 // per lane: 8 with two tasks, 4 with four (k = 4), 2 with two (k = 2).
 BatchKernel pick_shared(int r, int tasks_log2, bool vec) {
-  if (r == 8 && tasks_log2 == 1) return &batch_kernel<CodecF32, 8, unroll_for<8, 0>(), false, true, 1>;
+  if (r == 8 && tasks_log2 == 1) return &batch_kernel<CodecF32, 8, steps_in_flight(kPrecFP32, 8, 0), false, true, true, true, 1, 0>;
   if (r == 4 && tasks_log2 == 2)
-    return vec ? &batch_kernel<CodecF32, 4, unroll_for<4, 0>(), false, true, 2>
-               : &batch_kernel<CodecF32, 4, unroll_for<4, 0>(), false, false, 2>;
+    return vec ? &batch_kernel<CodecF32, 4, steps_in_flight(kPrecFP32, 4, 0), false, true, true, true, 2, 0>
+               : &batch_kernel<CodecF32, 4, steps_in_flight(kPrecFP32, 4, 0), false, false, true, true, 2, 0>;
   if (r == 2 && tasks_log2 == 1)
-    return vec ? &batch_kernel<CodecF32, 2, unroll_for<2, 0>(), false, true, 1>
-               : &batch_kernel<CodecF32, 2, unroll_for<2, 0>(), false, false, 1>;
+    return vec ? &batch_kernel<CodecF32, 2, steps_in_flight(kPrecFP32, 2, 0), false, true, true, true, 1, 0>
+               : &batch_kernel<CodecF32, 2, steps_in_flight(kPrecFP32, 2, 0), false, false, true, true, 1, 0>;
   return nullptr;
 }
 
