@@ -463,7 +463,8 @@ typedef struct {
                           (1 below k = 4; FP32: k for k <= 4).  With k / lanes >= 2 device x and y must be
                           16-byte aligned, except with lanes 0 and k <= 4 */
   int long_row_len;    /* rows longer than this are cut into chunks; 0: tuned, or 1024 for
-                          FP32, 256 below 2^22 nonzeros and for k >= 16, else 512 */
+                          FP32; else 256 below 2^22 nonzeros, 512 (256 for k >= 16) below
+                          2^25, 1024 above (FP64 from k = 8 on: 512 below 2^27) */
   int chunk;           /* entries per chunk; 0: long_row_len */
   int warps_per_block; /* 4 or 8; 0: tuned or 4 */
   int autotune;        /* 1: time candidate layouts on a sample of the batch and keep the fastest */

@@ -655,11 +655,21 @@ int default_tasks_log2(int k, int precision) {
 // Rows longer than this become chunks of it.  A chunk is one warp's work from
 // start to end, so where a batch is small, or its FP64 (or double-float) work per
 // entry large, long chunks run alone at the end: 0.5 M nonzeros, k = 32, FP64: 100
-// us at 1024, 45 at 256; 17 M: 1015 against 952.  Short ones cost partial sums
-// (17 M, k = 2, FP64: 103 at 512, 109 at 256).  FP32: 1024 always, as above.
+// us at 1024, 45 at 256; 17 M: 1015 against 952.  Short ones cost partial sums,
+// which is all that counts in a large batch.  FP32: 1024 always, as above.
+// us at 256, 512 and 1024 (lognormal rows; of 20 to 512 matrices):
+//            14 M nonzeros      60 M                141 M               537 M
+//   FP64 k=4   127  118  117     501  461  456      1126 1037 1017      4230 3883 3812
+//        k=8   218  214  229     902  882  895      2044 1995 1992      7742 7547 7475
+//        k=16  399  405  433    1715 1712 1732      3917 3884 3891     14890 14738 14648
+//   DF32 k=8   148  141  149     626  590  587      1417 1329 1307      5348 5012 4893
+//        k=16  263  261  279    1132 1097 1100      2571 2476 2459      9763 9374 9231
+//        k=32  468  473  500    2066 2047 2056      4705 4634 4615     17748 17459 17254
 int default_long_len(int k, int precision, int64_t nnz) {
   if (precision == kPrecFP32) return 1024;
-  return nnz < ((int64_t)1 << 22) || k >= 16 ? 256 : 512;
+  if (nnz < ((int64_t)1 << 22)) return 256;
+  if (nnz < ((int64_t)1 << 25)) return k >= 16 ? 256 : 512;
+  return precision == kPrecFP64 && k >= 8 && nnz < ((int64_t)1 << 27) ? 512 : 1024;
 }
 
 // Steps a row takes at most: a lane holds a whole row's right-hand sides at small
