@@ -189,6 +189,10 @@ int ilog2(int64_t v) {
   return l;
 }
 
+// Raised whenever the kernels, layouts or candidates change: choices timed on
+// others are not taken from the cache.
+constexpr int kTuneVersion = 1;
+
 // Cache key: the device and driver, the call shape and coarse features of the
 // batch (log2 buckets of its size and row lengths).
 std::string tune_key(const BatchSource& s, int k, int precision) {
@@ -206,8 +210,8 @@ std::string tune_key(const BatchSource& s, int k, int precision) {
       maxlen = std::max(maxlen, s.rp[(size_t)m][r + 1] - s.rp[(size_t)m][r]);
   }
   char buf[512];
-  std::snprintf(buf, sizeof(buf), "%s|sm%d|drv%d|k%d|p%d|n%d|r%d|z%d|a%d|m%d", prop.name, prop.multiProcessorCount,
-                drv, k, precision, ilog2(s.size()), ilog2(rows), ilog2(nnz), ilog2(rows ? 4 * nnz / rows : 0),
+  std::snprintf(buf, sizeof(buf), "v%d|%s|sm%d|drv%d|k%d|p%d|n%d|r%d|z%d|a%d|m%d", kTuneVersion, prop.name,
+                prop.multiProcessorCount, drv, k, precision, ilog2(s.size()), ilog2(rows), ilog2(nnz), ilog2(rows ? 4 * nnz / rows : 0),
                 ilog2(maxlen));
   for (char* c = buf; *c; ++c)
     if (*c == '"' || *c == '\n') *c = '_';
