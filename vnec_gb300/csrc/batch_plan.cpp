@@ -26,6 +26,13 @@ namespace {
 struct BatchDev {
   DeviceBuffer tasks, val, col, rowid, long_row, long_first, chunk_long, chunk_sum, chunk_count, xbuf, flag;
   BatchMatrix m;
+  void swap(BatchDev& o) {
+    for (auto p : {&BatchDev::tasks, &BatchDev::val, &BatchDev::col, &BatchDev::rowid, &BatchDev::long_row,
+                   &BatchDev::long_first, &BatchDev::chunk_long, &BatchDev::chunk_sum, &BatchDev::chunk_count,
+                   &BatchDev::xbuf, &BatchDev::flag})
+      (this->*p).swap(o.*p);
+    std::swap(m, o.m);
+  }
   int64_t bytes() const {
     return (int64_t)(tasks.bytes + val.bytes + col.bytes + rowid.bytes + long_row.bytes + long_first.bytes +
                      chunk_long.bytes + chunk_sum.bytes + chunk_count.bytes + xbuf.bytes + flag.bytes);
@@ -159,6 +166,49 @@ BatchHost* build_host(const BatchSource& s, const std::vector<int>& pick, int k,
   return batch_build((int)pick.size(), nr.data(), nc.data(), rp.data(), ci.data(), val.data(), k, prm);
 }
 
+// Default layout (measured on batches of 0.5 to 100 M nonzeros, lognormal rows,
+// every k and form).
+//
+// Right-hand sides per lane: FP64 and DF32 up to 4, as many as one lane loads in
+// 32 bytes, so the fewest lanes read each column and value (17 M nonzeros, FP64,
+// us at k = 2, 4, 8, 16, 32: 103, 146, 268, 496, 953 against 133, 182, 316, 598,
+// 1100 with half as many).  The FP32 form keeps one per lane up to k = 4, then 4:
+// the slots a row is spread over decide how its FP32 sums round.  It gets its wide
+// loads from several tasks per warp (default_tasks_log2).
+int default_lanes(int k, int precision) {
+  return precision == kPrecFP32 ? (k >= 8 ? k / 4 : k) : k / std::min(k, 4);
+}
+int default_tasks_log2(int k, int precision) {
+  return precision != kPrecFP32 || k == 1 ? 0 : k == 4 ? 2 : 1;
+}
+
+// Rows longer than this become chunks of it.  A chunk is one warp's work from
+// start to end, so where a batch is small, or its FP64 (or double-float) work per
+// entry large, long chunks run alone at the end: 0.5 M nonzeros, k = 32, FP64: 100
+// us at 1024, 45 at 256; 17 M: 1015 against 952.  Short ones cost partial sums,
+// which is all that counts in a large batch.  FP32: 1024 always, as above.
+// us at 256, 512 and 1024 (lognormal rows; of 20 to 512 matrices):
+//            14 M nonzeros      60 M                141 M               537 M
+//   FP64 k=4   127  118  117     501  461  456      1126 1037 1017      4230 3883 3812
+//        k=8   218  214  229     902  882  895      2044 1995 1992      7742 7547 7475
+//        k=16  399  405  433    1715 1712 1732      3917 3884 3891     14890 14738 14648
+//   DF32 k=8   148  141  149     626  590  587      1417 1329 1307      5348 5012 4893
+//        k=16  263  261  279    1132 1097 1100      2571 2476 2459      9763 9374 9231
+//        k=32  468  473  500    2066 2047 2056      4705 4634 4615     17748 17459 17254
+int default_long_len(int k, int precision, int64_t nnz) {
+  if (precision == kPrecFP32) return 1024;
+  if (nnz < ((int64_t)1 << 22)) return 256;
+  if (nnz < ((int64_t)1 << 25)) return k >= 16 ? 256 : 512;
+  return precision == kPrecFP64 && k >= 8 && nnz < ((int64_t)1 << 27) ? 512 : 1024;
+}
+
+// Steps a row takes at most: a lane holds a whole row's right-hand sides at small
+// k, so a small batch fills the GPU only with rows split over more slots (0.8 M
+// nonzeros, k = 2, FP64: 18.6 us at 32 steps, 12.5 at 16; 3.5 M: 39 against 31).
+int default_steps(int k, int precision, int64_t nnz) {
+  return precision != kPrecFP32 && k <= 8 && nnz < ((int64_t)1 << 22) ? 16 : 32;
+}
+
 // ---------------------------------------------------------------------------
 // Autotuner.
 // ---------------------------------------------------------------------------
@@ -172,7 +222,17 @@ struct TuneChoice {
   // window (k = 32: DF32 27.2 -> 17.6 ms, FP32 11.6 -> 8.2 ms, FP64 31.3 ->
   // 29.4 ms per call).  The autotuner decides it on the whole batch.
   bool per_task = true;
+  int tasks_log2 = 0;  // BatchMatrix::tasks_log2
 };
+
+// The layout of a plan that is not tuned.
+TuneChoice default_choice(int k, int precision, int64_t nnz) {
+  TuneChoice c;
+  c.lanes = default_lanes(k, precision);
+  c.long_len = default_long_len(k, precision, nnz);
+  c.tasks_log2 = default_tasks_log2(k, precision);
+  return c;
+}
 
 std::mutex g_tune_mu;
 std::map<std::string, TuneChoice>& tune_cache() {
@@ -191,7 +251,7 @@ int ilog2(int64_t v) {
 
 // Raised whenever the kernels, layouts or candidates change: choices timed on
 // others are not taken from the cache.
-constexpr int kTuneVersion = 1;
+constexpr int kTuneVersion = 2;
 
 // Cache key: the device and driver, the call shape and coarse features of the
 // batch (log2 buckets of its size and row lengths).
@@ -220,7 +280,8 @@ std::string tune_key(const BatchSource& s, int k, int precision) {
 
 // Optional persistent cache: one JSON object per line in the file named by
 // VNEC_TUNE_CACHE, {"key": "...", "lanes": L, "long_row_len": N, "warps_per_block": W,
-// "deep_unroll": D, "dispatch": 1 (persistent warps) or 2 (one warp per task)}.
+// "deep_unroll": D, "dispatch": 1 (persistent warps) or 2 (one warp per task),
+// "tasks_log2": T}.
 bool cache_file_lookup(const std::string& key, TuneChoice* c) {
   const char* path = std::getenv("VNEC_TUNE_CACHE");
   if (!path || !*path) return false;
@@ -234,8 +295,8 @@ bool cache_file_lookup(const std::string& key, TuneChoice* c) {
     int dispatch = 0;
     if (std::sscanf(line,
                     "{\"key\": \"%599[^\"]\", \"lanes\": %d, \"long_row_len\": %d, \"warps_per_block\": %d, "
-                    "\"deep_unroll\": %d, \"dispatch\": %d}",
-                    k, &t.lanes, &t.long_len, &t.wpb, &t.deep, &dispatch) == 6 &&
+                    "\"deep_unroll\": %d, \"dispatch\": %d, \"tasks_log2\": %d}",
+                    k, &t.lanes, &t.long_len, &t.wpb, &t.deep, &dispatch, &t.tasks_log2) == 7 &&
         key == k) {
       t.per_task = dispatch == 2;
       *c = t;
@@ -253,8 +314,8 @@ void cache_file_store(const std::string& key, const TuneChoice& c) {
   if (!f) return;
   std::fprintf(f,
                "{\"key\": \"%s\", \"lanes\": %d, \"long_row_len\": %d, \"warps_per_block\": %d, "
-               "\"deep_unroll\": %d, \"dispatch\": %d}\n",
-               key.c_str(), c.lanes, c.long_len, c.wpb, c.deep, c.per_task ? 2 : 1);
+               "\"deep_unroll\": %d, \"dispatch\": %d, \"tasks_log2\": %d}\n",
+               key.c_str(), c.lanes, c.long_len, c.wpb, c.deep, c.per_task ? 2 : 1, c.tasks_log2);
   std::fclose(f);
 }
 
@@ -283,6 +344,7 @@ struct TuneRun {
   std::vector<TuneChoice> cand;
   std::vector<float> ms;
   int best = -1;
+  bool whole = false;  // the sample was the whole batch
 };
 
 float median_ms(std::vector<float> v) {
@@ -290,10 +352,15 @@ float median_ms(std::vector<float> v) {
   return v.empty() ? 0.f : v[v.size() / 2];
 }
 
-bool autotune(const BatchSource& s, int k, int precision, const SpB_VNEC_batch_options_ext* o, TuneRun* run) {
+// The layout a plan takes when nothing is tuned is among the candidates: its chunk
+// length and step limit, and its tasks per warp wherever its lanes run in mode 0.
+bool autotune(const BatchSource& s, int k, int precision, int64_t nnz, const SpB_VNEC_batch_options_ext* o,
+              TuneRun* run) {
+  const TuneChoice def = default_choice(k, precision, nnz);
   std::vector<int> lanes_c, long_c{256, 1024, 4096}, wpb_c{4, 8}, deep_c{0, 1, 2};
   for (int L = 1; L <= 32; L <<= 1)
     if (batch_supported(k, L)) lanes_c.push_back(L);
+  if (std::find(long_c.begin(), long_c.end(), def.long_len) == long_c.end()) long_c.push_back(def.long_len);
   if (o->lanes > 0) lanes_c = {o->lanes};
   if (o->long_row_len > 0) long_c = {o->long_row_len};
   if (o->warps_per_block > 0) wpb_c = {o->warps_per_block};
@@ -302,6 +369,7 @@ bool autotune(const BatchSource& s, int k, int precision, const SpB_VNEC_batch_o
   if (o->dispatch == 1) disp_c = {0};
   if (o->dispatch == 2) disp_c = {1};
   const std::vector<int> pick = tune_sample(s, (int64_t)48 << 20);
+  run->whole = (int)pick.size() == s.size();
   TimingStream ts;
   if (!ts.create()) {
     set_error("batch autotune: cannot create a stream or events");
@@ -318,7 +386,7 @@ bool autotune(const BatchSource& s, int k, int precision, const SpB_VNEC_batch_o
       prm.long_len = ll;
       prm.chunk = o->chunk > 0 ? o->chunk : ll;
       if (o->window_rows > 0) prm.window_rows = o->window_rows;
-      if (o->max_steps > 0) prm.max_steps = o->max_steps;
+      prm.max_steps = o->max_steps > 0 ? o->max_steps : default_steps(k, precision, nnz);
       BatchHost* h = build_host(s, pick, k, prm);
       if (!h) continue;
       const BatchHostView hv = batch_view(h);
@@ -341,27 +409,36 @@ bool autotune(const BatchSource& s, int k, int precision, const SpB_VNEC_batch_o
           // (persistent only if it wins by more than 3 %).
           d.m.mode = deep;
           d.m.grid = batch_grid(precision, k / L, wpb, d.m.mode);
-          float best_ms[2] = {0.f, 0.f};
-          for (int pt : disp_c) {
-            d.m.per_task = pt != 0;
-            std::vector<float> t;
-            for (int rep = 0; rep < 7 && ok; ++rep) {
-              ok = VNEC_CUDA(cudaEventRecord(e0, st)) && batch_spmm(d.m, X.as<double>(), Y.as<double>(), st) &&
-                   VNEC_CUDA(cudaEventRecord(e1, st)) && VNEC_CUDA(cudaEventSynchronize(e1));
-              float ms = 0.f;
-              if (ok && rep >= 2 && VNEC_CUDA(cudaEventElapsedTime(&ms, e0, e1))) t.push_back(ms);
+          TuneChoice c{L, ll, wpb, deep};
+          float c_ms = 0.f;
+          std::vector<int> tl_c{0};
+          if (o->lanes == 0 && L == def.lanes && deep == 0 && def.tasks_log2 > 0) tl_c.push_back(def.tasks_log2);
+          for (int tl : tl_c) {
+            d.m.tasks_log2 = tl;
+            float best_ms[2] = {0.f, 0.f};
+            for (int pt : disp_c) {
+              d.m.per_task = pt != 0;
+              std::vector<float> t;
+              for (int rep = 0; rep < 7 && ok; ++rep) {
+                ok = VNEC_CUDA(cudaEventRecord(e0, st)) && batch_spmm(d.m, X.as<double>(), Y.as<double>(), st) &&
+                     VNEC_CUDA(cudaEventRecord(e1, st)) && VNEC_CUDA(cudaEventSynchronize(e1));
+                float ms = 0.f;
+                if (ok && rep >= 2 && VNEC_CUDA(cudaEventElapsedTime(&ms, e0, e1))) t.push_back(ms);
+              }
+              if (!ok) break;
+              best_ms[pt] = median_ms(t);
             }
             if (!ok) break;
-            best_ms[pt] = median_ms(t);
+            const bool per_task = disp_c.size() == 2 ? !(best_ms[0] < 0.97f * best_ms[1]) : disp_c[0] != 0;
+            if (c_ms == 0.f || best_ms[per_task ? 1 : 0] < c_ms) {
+              c_ms = best_ms[per_task ? 1 : 0];
+              c.per_task = per_task;
+              c.tasks_log2 = tl;
+            }
           }
           if (!ok) break;
-          TuneChoice c{L, ll, wpb, deep};
-          if (disp_c.size() == 2)
-            c.per_task = !(best_ms[0] < 0.97f * best_ms[1]);
-          else
-            c.per_task = disp_c[0] != 0;
           run->cand.push_back(c);
-          run->ms.push_back(best_ms[c.per_task ? 1 : 0]);
+          run->ms.push_back(c_ms);
         }
         if (!ok) break;
       }
@@ -382,8 +459,8 @@ bool autotune(const BatchSource& s, int k, int precision, const SpB_VNEC_batch_o
 
 // Times the uploaded plan with persistent warps and with one warp per task
 // (median of 3 calls after one warm-up each, on scratch X and Y) and keeps
-// persistent warps only when they win by more than 3 %.
-bool whole_batch_dispatch(BatchMatrix& m, int64_t n_rows, int64_t n_cols, int k, bool* per_task) {
+// persistent warps only when they win by more than 3 %; *ms is the kept time.
+bool whole_batch_dispatch(BatchMatrix& m, int64_t n_rows, int64_t n_cols, int k, bool* per_task, float* ms) {
   TimingStream ts;
   DeviceBuffer X, Y;
   if (!ts.create()) {
@@ -400,12 +477,13 @@ bool whole_batch_dispatch(BatchMatrix& m, int64_t n_rows, int64_t n_cols, int k,
       if (!VNEC_CUDA(cudaEventRecord(ts.e0, ts.s)) || !batch_spmm(m, X.as<double>(), Y.as<double>(), ts.s) ||
           !VNEC_CUDA(cudaEventRecord(ts.e1, ts.s)) || !VNEC_CUDA(cudaEventSynchronize(ts.e1)))
         return false;
-      float ms = 0.f;
-      if (rep >= 1 && VNEC_CUDA(cudaEventElapsedTime(&ms, ts.e0, ts.e1))) t.push_back(ms);
+      float one = 0.f;
+      if (rep >= 1 && VNEC_CUDA(cudaEventElapsedTime(&one, ts.e0, ts.e1))) t.push_back(one);
     }
     med[pt] = median_ms(t);
   }
   *per_task = !(med[0] < 0.97f * med[1]);
+  *ms = med[*per_task ? 1 : 0];
   return true;
 }
 
@@ -614,73 +692,31 @@ struct BatchPlan final : Plan {
 // Host-call parts: about `n_parts` groups of whole windows with equal
 // entries; part i copies in the X rows of the matrices its rows belong to that
 // earlier parts did not (the last part takes every remaining X row).
-void plan_parts(BatchPlan* p, const BatchHostView& hv, int n_parts) {
-  p->parts.clear();
-  if (hv.num_windows < 2 || n_parts < 2) return;
-  const int64_t W = p->prm.window_rows;
-  const int n = (int)p->row_off.size() - 1;
+std::vector<BatchPlan::Part> plan_parts(const BatchPlan& p, const BatchHostView& hv, int n_parts) {
+  std::vector<BatchPlan::Part> parts;
+  if (hv.num_windows < 2 || n_parts < 2) return parts;
+  const int64_t W = p.prm.window_rows;
+  const int n = (int)p.row_off.size() - 1;
   int64_t w0 = 0, c_done = 0;
   for (int i = 1; i <= n_parts && w0 < hv.num_windows; ++i) {
     const int64_t target = hv.win_entry[hv.num_windows] * i / n_parts;
     int64_t w1 = w0 + 1;
     while (w1 < hv.num_windows && hv.win_entry[w1] < target) ++w1;
     if (i == n_parts) w1 = hv.num_windows;
-    const int64_t r0 = w0 * W, r1 = std::min<int64_t>(p->n_rows, w1 * W);
+    const int64_t r0 = w0 * W, r1 = std::min<int64_t>(p.n_rows, w1 * W);
     int64_t c1 = c_done;
     if (w1 == hv.num_windows) {
-      c1 = p->n_cols;
+      c1 = p.n_cols;
     } else if (r1 > r0) {
       // matrix of the part's last row: the last m with row_off[m] <= r1 - 1
-      const int m = (int)(std::upper_bound(p->row_off.begin(), p->row_off.end(), r1 - 1) - p->row_off.begin()) - 1;
-      c1 = std::max(c_done, p->col_off[(size_t)std::min(m + 1, n)]);
+      const int m = (int)(std::upper_bound(p.row_off.begin(), p.row_off.end(), r1 - 1) - p.row_off.begin()) - 1;
+      c1 = std::max(c_done, p.col_off[(size_t)std::min(m + 1, n)]);
     }
-    p->parts.push_back(BatchPlan::Part{hv.win_task[w0], hv.win_task[w1], r0, r1, c_done, c1});
+    parts.push_back(BatchPlan::Part{hv.win_task[w0], hv.win_task[w1], r0, r1, c_done, c1});
     c_done = c1;
     w0 = w1;
   }
-}
-
-// Default layout (measured on batches of 0.5 to 100 M nonzeros, lognormal rows,
-// every k and form).
-//
-// Right-hand sides per lane: FP64 and DF32 up to 4, as many as one lane loads in
-// 32 bytes, so the fewest lanes read each column and value (17 M nonzeros, FP64,
-// us at k = 2, 4, 8, 16, 32: 103, 146, 268, 496, 953 against 133, 182, 316, 598,
-// 1100 with half as many).  The FP32 form keeps one per lane up to k = 4, then 4:
-// the slots a row is spread over decide how its FP32 sums round.  It gets its wide
-// loads from several tasks per warp (default_tasks_log2).
-int default_lanes(int k, int precision) {
-  return precision == kPrecFP32 ? (k >= 8 ? k / 4 : k) : k / std::min(k, 4);
-}
-int default_tasks_log2(int k, int precision) {
-  return precision != kPrecFP32 || k == 1 ? 0 : k == 4 ? 2 : 1;
-}
-
-// Rows longer than this become chunks of it.  A chunk is one warp's work from
-// start to end, so where a batch is small, or its FP64 (or double-float) work per
-// entry large, long chunks run alone at the end: 0.5 M nonzeros, k = 32, FP64: 100
-// us at 1024, 45 at 256; 17 M: 1015 against 952.  Short ones cost partial sums,
-// which is all that counts in a large batch.  FP32: 1024 always, as above.
-// us at 256, 512 and 1024 (lognormal rows; of 20 to 512 matrices):
-//            14 M nonzeros      60 M                141 M               537 M
-//   FP64 k=4   127  118  117     501  461  456      1126 1037 1017      4230 3883 3812
-//        k=8   218  214  229     902  882  895      2044 1995 1992      7742 7547 7475
-//        k=16  399  405  433    1715 1712 1732      3917 3884 3891     14890 14738 14648
-//   DF32 k=8   148  141  149     626  590  587      1417 1329 1307      5348 5012 4893
-//        k=16  263  261  279    1132 1097 1100      2571 2476 2459      9763 9374 9231
-//        k=32  468  473  500    2066 2047 2056      4705 4634 4615     17748 17459 17254
-int default_long_len(int k, int precision, int64_t nnz) {
-  if (precision == kPrecFP32) return 1024;
-  if (nnz < ((int64_t)1 << 22)) return 256;
-  if (nnz < ((int64_t)1 << 25)) return k >= 16 ? 256 : 512;
-  return precision == kPrecFP64 && k >= 8 && nnz < ((int64_t)1 << 27) ? 512 : 1024;
-}
-
-// Steps a row takes at most: a lane holds a whole row's right-hand sides at small
-// k, so a small batch fills the GPU only with rows split over more slots (0.8 M
-// nonzeros, k = 2, FP64: 18.6 us at 32 steps, 12.5 at 16; 3.5 M: 39 against 31).
-int default_steps(int k, int precision, int64_t nnz) {
-  return precision != kPrecFP32 && k <= 8 && nnz < ((int64_t)1 << 22) ? 16 : 32;
+  return parts;
 }
 
 // A k = 1 batch as one sliced plan: the block-diagonal concatenation (matrix
@@ -810,68 +846,96 @@ std::unique_ptr<Plan> build_batch(int n, const CsrView* mats, int k, const SpB_V
     return p;
   }
 
-  TuneChoice choice;
-  choice.lanes = o.lanes > 0 ? o.lanes : default_lanes(k, o.precision);
-  choice.long_len = o.long_row_len > 0 ? o.long_row_len : default_long_len(k, o.precision, p->nnz);
+  const TuneChoice def = default_choice(k, o.precision, p->nnz);
+  const bool free_layout =
+      o.lanes == 0 && o.long_row_len == 0 && o.warps_per_block == 0 && o.unroll == 0 && o.dispatch == 0;
+  TuneChoice choice = def;
+  if (o.lanes > 0) choice.lanes = o.lanes;
+  if (o.long_row_len > 0) choice.long_len = o.long_row_len;
   if (o.warps_per_block > 0) choice.wpb = o.warps_per_block;
   if (o.unroll > 0) choice.deep = o.unroll - 1;
-  bool fresh = false;  // layout tuned here: the dispatch is then decided on the whole batch
+  if (o.lanes > 0 || choice.deep != 0) choice.tasks_log2 = 0;
+  bool fresh = false;  // layout tuned here: what the sample cannot show is then timed on the whole batch
   std::string key;
   if (o.autotune) {
     key = tune_key(src, k, o.precision);
     bool hit = false;
-    if (o.lanes == 0 && o.long_row_len == 0 && o.warps_per_block == 0 && o.unroll == 0 &&
-        o.dispatch == 0) {
+    if (free_layout) {
       std::lock_guard<std::mutex> g(g_tune_mu);
       auto it = tune_cache().find(key);
       if (it != tune_cache().end()) {
         choice = it->second;
         hit = true;
       } else if (cache_file_lookup(key, &choice)) {
-        tune_cache()[key] = choice;
-        hit = batch_supported(k, choice.lanes);
+        hit = batch_supported(k, choice.lanes) &&
+              (choice.tasks_log2 == 0 || (choice.tasks_log2 == def.tasks_log2 && choice.lanes == def.lanes && choice.deep == 0));
+        if (hit) tune_cache()[key] = choice;
       }
     }
     if (!hit) {
-      if (!autotune(src, k, o.precision, &o, &p->tuning)) return nullptr;
+      if (!autotune(src, k, o.precision, p->nnz, &o, &p->tuning)) return nullptr;
       choice = p->tuning.cand[(size_t)p->tuning.best];
       fresh = true;
     }
   }
-  p->prm.lanes = choice.lanes;
-  p->prm.long_len = choice.long_len;
-  p->prm.chunk = o.chunk > 0 ? o.chunk : choice.long_len;
   if (o.window_rows > 0) p->prm.window_rows = o.window_rows;
-  p->prm.max_steps = o.max_steps > 0 ? o.max_steps : o.autotune ? p->prm.max_steps : default_steps(k, o.precision, p->nnz);
+  p->prm.max_steps = o.max_steps > 0 ? o.max_steps : default_steps(k, o.precision, p->nnz);
   p->any_alignment = o.lanes == 0 && k <= 4;
   std::vector<int> all((size_t)n);
   for (int m = 0; m < n; ++m) all[(size_t)m] = m;
-  BatchHost* h = build_host(src, all, k, p->prm);
-  if (!h) {
-    set_error("batch: more than 2^31 rows, columns or layout entries");
-    return nullptr;
-  }
-  const bool ok = upload_batch(h, k, o.precision, choice.wpb, choice.deep, &p->d);
-  if (ok && fresh && o.dispatch == 0) {
-    // The sample the layout was tuned on holds a fraction of the batch, so
-    // how far the persistent warps' drift spreads the rows of X they gather
-    // shows only on the whole batch: time both dispatches on it.
-    if (!whole_batch_dispatch(p->d.m, p->n_rows, p->n_cols, k, &choice.per_task)) {
-      batch_free(h);
-      return nullptr;
+  // The whole batch in choice c's layout, on the device, and its host-call parts.
+  auto build = [&](const TuneChoice& c, BatchDev* d, std::vector<BatchPlan::Part>* parts) {
+    BatchParams prm = p->prm;
+    prm.lanes = c.lanes;
+    prm.long_len = c.long_len;
+    prm.chunk = o.chunk > 0 ? o.chunk : c.long_len;
+    BatchHost* h = build_host(src, all, k, prm);
+    if (!h) {
+      set_error("batch: more than 2^31 rows, columns or layout entries");
+      return false;
+    }
+    const bool ok = upload_batch(h, k, o.precision, c.wpb, c.deep, d);
+    d->m.tasks_log2 = c.tasks_log2;
+    if (ok) *parts = plan_parts(*p, batch_view(h), o.host_parts > 0 ? o.host_parts : 8);
+    batch_free(h);
+    return ok;
+  };
+  if (!build(choice, &p->d, &p->parts)) return nullptr;
+  if (fresh && o.dispatch == 0) {
+    // The sample the layout was tuned on holds a fraction of the batch, so how far
+    // the persistent warps' drift spreads the rows of X they gather, and what X no
+    // longer fits in L2 costs, shows only on the whole batch: time both dispatches
+    // on it, and the untuned layout beside the sample's best (512 matrices, DF32,
+    // k = 16: 9.73 ms by the sample's order, 9.23 untuned).
+    float ms = 0.f, def_ms = 0.f;
+    if (!whole_batch_dispatch(p->d.m, p->n_rows, p->n_cols, k, &choice.per_task, &ms)) return nullptr;
+    if (free_layout && !p->tuning.whole) {
+      TuneChoice other = def;
+      BatchDev d;
+      std::vector<BatchPlan::Part> parts;
+      // (Where there is no room for a second layout, the tuned one stands.)
+      if (build(other, &d, &parts) &&
+          whole_batch_dispatch(d.m, p->n_rows, p->n_cols, k, &other.per_task, &def_ms) && def_ms < ms) {
+        p->d.swap(d);
+        p->parts.swap(parts);
+        choice = other;
+        for (size_t i = 0; i < p->tuning.cand.size(); ++i) {
+          const TuneChoice& c = p->tuning.cand[i];
+          if (c.lanes == def.lanes && c.long_len == def.long_len && c.wpb == def.wpb && c.deep == def.deep)
+            p->tuning.best = (int)i;
+        }
+      }
     }
   }
-  if (fresh && o.lanes == 0 && o.long_row_len == 0 && o.warps_per_block == 0 && o.unroll == 0 &&
-      o.dispatch == 0) {
+  if (fresh && free_layout) {
     std::lock_guard<std::mutex> g(g_tune_mu);
     tune_cache()[key] = choice;
     cache_file_store(key, choice);
   }
-  if (o.lanes == 0 && !o.autotune && choice.deep == 0) p->d.m.tasks_log2 = default_tasks_log2(k, o.precision);
+  p->prm.lanes = choice.lanes;
+  p->prm.long_len = choice.long_len;
+  p->prm.chunk = o.chunk > 0 ? o.chunk : choice.long_len;
   p->d.m.per_task = o.dispatch == 0 ? choice.per_task : o.dispatch == 2;
-  if (ok) plan_parts(p.get(), batch_view(h), o.host_parts > 0 ? o.host_parts : 8);
-  batch_free(h);
-  if (!ok) return nullptr;
   return p;
 }
 

@@ -7,6 +7,7 @@
 #include <cstdint>
 #include <cstring>
 #include <string>
+#include <utility>
 
 namespace vnec {
 
@@ -92,6 +93,10 @@ struct DeviceBuffer {
   ~DeviceBuffer() { release(); }
   bool alloc(size_t n);
   void release();
+  void swap(DeviceBuffer& o) {
+    std::swap(ptr, o.ptr);
+    std::swap(bytes, o.bytes);
+  }
   template <typename T> T* as() const { return static_cast<T*>(ptr); }
 };
 
