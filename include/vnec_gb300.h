@@ -173,7 +173,7 @@ typedef struct {
                             y n_cols; any kernel, built on A's transpose */
   int host_parts;        /* sliced FP64 plans: host-vector calls run in this many parts so
                             that y copies overlap the SpMV (0: 4 where y is page-locked
-                            and of 12 MB at least, else one; 1: one part) */
+                            and of 10 MB at least, 7 MB of FP32 values, else one; 1: one part) */
   int column_deltas;     /* sliced: store the columns of one-row-per-lane groups as 16-bit
                             deltas where the gaps allow (0: on unless a hot-column window
                             is used, -1: off) */

@@ -1,7 +1,8 @@
 /* A stand-in for the CUDA runtime calls that the library's host code makes, to be
  * preloaded on a machine without a GPU: device memory is host memory, launches do
- * nothing.  FAKE_FAIL names the calls that fail ("hostalloc", "hostmap").  The 7th
- * argument of a chained launch with 14 arguments or more (y of the sliced kernel) is
+ * nothing.  FAKE_FAIL names the calls that fail ("hostalloc", "hostmap"); with
+ * FAKE_LOCKED set, callers' arrays count as page-locked.  The 7th
+ * argument of a chained launch (y of the sliced kernel, the only one that the tests make) is
  * printed by its kind: "null", "mapped" (from cudaHostAlloc) or "device". */
 #include <cuda_runtime_api.h>
 #include <stdio.h>
@@ -45,6 +46,12 @@ cudaError_t cudaMemset(void* p, int v, size_t n) { memset(p, v, n); return cudaS
 cudaError_t cudaMemsetAsync(void* p, int v, size_t n, cudaStream_t s) { (void)s; memset(p, v, n); return cudaSuccess; }
 cudaError_t cudaGetDevice(int* d) { *d = 0; return cudaSuccess; }
 cudaError_t cudaDeviceGetAttribute(int* v, enum cudaDeviceAttr a, int d) { (void)a; (void)d; *v = 152; return cudaSuccess; }
+cudaError_t cudaPointerGetAttributes(struct cudaPointerAttributes* a, const void* p) {
+  (void)p;
+  memset(a, 0, sizeof(*a));
+  a->type = getenv("FAKE_LOCKED") ? cudaMemoryTypeHost : cudaMemoryTypeUnregistered;
+  return cudaSuccess;
+}
 cudaError_t cudaGetLastError(void) { return cudaSuccess; }
 const char* cudaGetErrorString(cudaError_t e) { (void)e; return "fake error"; }
 cudaError_t cudaFuncSetAttribute(const void* f, enum cudaFuncAttribute a, int v) { (void)f; (void)a; (void)v; return cudaSuccess; }

@@ -98,12 +98,14 @@ struct SlicedPlan final : Plan {
   // By default a call is split only where that pays: y page-locked, so that its
   // copies run beside the kernels (a copy to pageable memory holds up the next
   // part's launch: 200,000 rows 71 us whole, 144 in 8 parts; 16 M rows 1.86
-  // against 2.05 ms), and of 12 MB at least (page-locked, whole against 4 and 8
-  // parts: 200,000 rows 47, 63 and 62 us; 1.6 M 204, 197, 208; 16 M 1739, 1440,
-  // 1461).
+  // against 2.05 ms), and long enough: of 10 MB at least, or of 7 MB of FP32 values,
+  // whose kernels take longer beside their copies (page-locked, whole against 4 and
+  // 8 parts, us: FP64 9 MB 147, 154 and 167, 11 MB 180, 173 and 183, 16 MB 247, 230
+  // and 241; FP32 type 5 MB 107, 113 and 125, 9 MB 180, 162 and 170, 11 MB 216, 187
+  // and 196).
   bool split_pays(const void* h_y) const {
     if (parts_asked) return true;
-    if ((type == SpB_FP64 ? 8 : 4) * n_rows < ((int64_t)12 << 20)) return false;
+    if (type == SpB_FP64 ? 8 * n_rows < ((int64_t)10 << 20) : 4 * n_rows < ((int64_t)7 << 20)) return false;
     cudaPointerAttributes at{};
     if (cudaPointerGetAttributes(&at, h_y) != cudaSuccess) {
       cudaGetLastError();
