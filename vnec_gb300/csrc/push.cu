@@ -9,11 +9,11 @@
 //
 // Split of the work.  A frontier of a power-law graph mixes columns of one
 // entry with hubs of tens of thousands, so neither columns nor warps per
-// column balance.  The entries of x are dealt out to chunks of kChunk (entry
-// i * chunks + c to chunk c, so that neighbouring hubs fall to different
-// chunks); `parts` blocks share a chunk: each scans the chunk's column lengths
-// into shared memory and takes an equal share of their sum, cut into one
-// contiguous run per warp.  The scan is repeated by the chunk's blocks instead
+// column balance (plans of short columns only: push_columns_kernel).  The
+// entries of x are dealt out to chunks of kChunk (entry i * chunks + c to chunk
+// c, so that neighbouring hubs fall to different chunks); `parts` blocks share a
+// chunk: each scans the chunk's column lengths into shared memory and takes an
+// equal share of their sum, cut into one contiguous run per warp.  The scan is repeated by the chunk's blocks instead
 // of handed from one launch to the next: it is three loads a thread, and calls
 // on several streams share no scratch.
 // What bounds it now: the L2's atomics, the ones on the lines of the hub rows
@@ -43,6 +43,10 @@ constexpr int kUnroll = 4;   // column entries in flight per lane
 // Blocks wanted in all: enough that a chunk with a hub column of tens of
 // thousands of entries is shared by many (half or twice as many: within 5%).
 constexpr long long kBlocks = 152LL * 16;
+// ... but no more than give each at least this many entries, were the frontier's
+// columns average and one the longest: every part scans its chunk anew (R-MAT
+// 2^13, dense x: 19.6 -> 13.5 us; 1,000 vertices of 2^18: 10.1 -> 8.3).
+constexpr long long kPartEntries = 256;
 
 template <typename V>
 __global__ void __launch_bounds__(kChunk)
@@ -127,12 +131,58 @@ push_kernel(long long nx, const int32_t* __restrict__ idx, const V* __restrict__
   }
 }
 
+// One warp per column, for plans whose columns are all short: without hubs there
+// is nothing to balance, and a warp has its column's entries after two dependent
+// loads, where the scan costs a block four and two barriers.
+template <typename V>
+__global__ void __launch_bounds__(kChunk)
+push_columns_kernel(long long nx, const int32_t* __restrict__ idx, const V* __restrict__ xval,
+                    const int64_t* __restrict__ cp, const int32_t* __restrict__ row, const V* __restrict__ val,
+                    long long n_cols, V* __restrict__ y, int* __restrict__ status) {
+  const int lane = threadIdx.x & 31;
+  const long long nw = (long long)gridDim.x * kWarps;
+  for (long long w = (long long)blockIdx.x * kWarps + (threadIdx.x >> 5); w < nx; w += nw) {
+    const long long j = idx ? (long long)__ldg(idx + w) : w;
+    if (j < 0 || j >= n_cols) {
+      if (lane == 0) atomicExch(status, 1);
+      continue;
+    }
+    const V xj = __ldg(xval + w);
+    if (xj == V(0)) continue;
+    const long long b = __ldg(cp + j), e = __ldg(cp + j + 1);
+    for (long long p = b + lane; p < e; p += 32) atomicAdd(y + __ldg(row + p), __ldcs(val + p) * xj);
+  }
+}
+
+// Columns one by one where none is longer than kShortColumn and there are enough of
+// them to fill the GPU (else a chunk's blocks share a column: 33 columns of 300
+// entries 10.3 us by warps, 8.3 shared).  The more columns, the more the scan
+// gets out of full warps, and the sooner so the shorter they are.  us, shared ->
+// by warps, FP64: 20 entries a column (lognormal rows), 4,000 columns 14.2 -> 8.3,
+// 50,000 22.7 -> 16.4; 9 entries, 6,000 14.5 -> 8.0, 75,000 18.6 -> 18.5, 300,000
+// 32.8 -> 47; 33 entries, 200,000 34.9 -> 47; 100 entries, 25,000 28.7 -> 22.6,
+// 100,000 74.6 -> 63.5; 1 entry, 1,000 10.3 -> 9.7, 40,000 11.5 -> 13.6.
+constexpr int64_t kShortColumn = 512;
+bool by_columns(const PushMatrix& m, long long nx) {
+  if (m.longest > kShortColumn || nx < 256) return false;
+  return m.nnz >= 64 * m.n_cols || nx <= 16384 || (nx <= 131072 && m.nnz >= 8 * m.n_cols);
+}
+
 template <typename V>
 bool launch(const PushMatrix& m, long long nx, const int32_t* idx, const void* xval, void* y, cudaStream_t s) {
   if (m.n_rows > 0 && !VNEC_CUDA(cudaMemsetAsync(y, 0, sizeof(V) * (size_t)m.n_rows, s))) return false;
   if (nx <= 0) return true;
+  if (by_columns(m, nx)) {
+    const long long grid = std::min<long long>((nx + kWarps - 1) / kWarps, 152LL * 32);
+    push_columns_kernel<V><<<(unsigned)grid, kChunk, 0, s>>>(nx, idx, static_cast<const V*>(xval), m.col_ptr, m.row,
+                                                            static_cast<const V*>(m.val), m.n_cols,
+                                                            static_cast<V*>(y), m.status);
+    return VNEC_CUDA(cudaGetLastError());
+  }
   const long long chunks = (nx + kChunk - 1) / kChunk;
-  const long long parts = std::min<long long>(std::max<long long>(kBlocks / chunks, 1), 64);
+  const long long most = kChunk * (m.nnz / std::max<long long>(m.n_cols, 1) + 1) + m.longest;
+  const long long parts =
+      std::max<long long>(1, std::min<long long>({kBlocks / chunks, 64, (most + kPartEntries - 1) / kPartEntries}));
   if (chunks * parts > 0x7fffffffLL) {
     set_error("SpMSpV: too many entries of x for one launch");
     return false;

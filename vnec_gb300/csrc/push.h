@@ -9,6 +9,7 @@ namespace vnec {
 
 struct PushMatrix {
   int64_t n_rows = 0, n_cols = 0, nnz = 0;
+  int64_t longest = 0;               // entries of the longest column
   const int64_t* col_ptr = nullptr;  // n_cols + 1
   const int32_t* row = nullptr;      // nnz row indices, increasing within a column
   const void* val = nullptr;         // nnz values (double or float)

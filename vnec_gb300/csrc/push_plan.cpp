@@ -74,6 +74,8 @@ std::unique_ptr<Plan> build_push(const CsrView& v, const SpB_VNEC_options_ext*) 
   p->m.n_rows = v.n_rows;
   p->m.n_cols = v.n_cols;
   p->m.nnz = v.nnz;
+  for (int64_t c = 0; c < v.n_cols; ++c)
+    p->m.longest = std::max(p->m.longest, t.row_ptr[(size_t)c + 1] - t.row_ptr[(size_t)c]);
   p->m.col_ptr = p->col_ptr.as<int64_t>();
   p->m.row = p->row.as<int32_t>();
   p->m.val = p->val.ptr;
