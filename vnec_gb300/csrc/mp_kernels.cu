@@ -435,7 +435,7 @@ bool launch_mp(const MpMatrix& m, const void* x, void* y, cudaStream_t s, cudaEv
   constexpr int kB = sizeof(V) == 8 ? 10 : 16;
   if (!(threads <= 128   ? launch_tiles<V, Off, 128, kB>(m, threads, x, y, s)
         : threads <= 256 ? launch_tiles<V, Off, 256, kB / 2>(m, threads, x, y, s)
-                         : launch_tiles<V, Off, kMaxTileThreads, 1>(m, threads, x, y, s)))
+                         : launch_tiles<V, Off, kMaxTileThreads, sizeof(V) == 8 ? 3 : 4>(m, threads, x, y, s)))
     return false;
   if (ev && !VNEC_CUDA(cudaEventRecord(ev[1], s))) return false;
   const int fb = 256;
