@@ -130,22 +130,34 @@ template <> struct Quad<float> {
   }
 };
 
-// One warp per task, U blocks of a lane in flight: their columns and values are
-// loaded together (the values do not wait for the columns), then their x, and the
-// last round is predicated instead of taking its blocks one by one.  U is 2 where
-// no task has more than kDenseShort blocks a lane, else kDenseAhead<V>.
-// What bounds it: latency (a block's columns, then its x; DRAM 40% busy before),
-// and for FP64 the FP64 pipe on filled-up blocks.  Against one block after the
-// other, us: FP32 blocks of 24 x 24, 500,003 rows, 18.6 -> 11.6 (U = 6 12.7); band
-// of 6, 3 M rows, FP64 49 -> 45 (4: 55), FP32 41 -> 22 (6: 35); stencil 100^3 68 -> 65
-// (4: 67) and 38 -> 31 (6: 32).  With longer tasks, where a chain of rounds ends the
-// call, U = 2 loses: lognormal rows FP64 108 (4) against 121, FP32 81 (6) against 89
-// (4 or 8: 74 against 65 at another size); 40,001 of them 34 against 49; 16 random
-// columns a row, FP64, 49 against 61; band of 129 43 against 46.
-template <typename V> constexpr int kDenseAhead = sizeof(V) == 8 ? 4 : 6;
+// One warp per task, U blocks of a lane in flight, the last round predicated instead
+// of taking its blocks one by one.  What bounds it: latency (a block's columns, then
+// its x), and for FP64 the FP64 pipe on filled-up blocks.  So what is loaded ahead is
+// weighed against the warps its registers cost, by the longest task of the plan:
+//   kDenseColumns: the columns of a round, values with each block's x (32 registers)
+//   kDenseValues:  a round's columns and values together (30 to 38)
+//   kDenseNext:    these, and the next round's columns (38 to 64)
+// us, one block after the other with four columns loaded -> kDenseColumns (U = 4, FP32
+// 6), kDenseValues (U = 2), kDenseNext (U = 2):
+//   FP64  2 random columns a row   35.1 -> 31.1, 40.8, 32.6   band of 6, 3 M rows  49.8 -> 43.5, 44.7, 49.7
+//         5                        31.0 -> 30.8, 41.7, 30.2   band of 16           12.4 -> 12.5, 10.7, 8.9
+//         9                        32.9 -> 33.2, 39.1, 33.0   blocks of 4          18.5 -> 13.5, 15.5, 17.6
+//         7                        29.2 -> 36.6, 37.2, 28.3   blocks of 32         16.6 -> 19.9, 16.6, 14.2
+//   FP32  7 random columns a row   24.7 -> 24.2, 26.5, 21.5   band of 6, 3 M rows  41.1 -> 27.1, 21.8, 27.2
+//         3                        26.8 -> 21.9, 23.6, 22.5   blocks of 24         10.3 -> 5.8, 5.2, 5.6
+//         8                        24.7 -> 25.1, 26.9, 21.5   blocks of 32         8.3 -> 7.2, 6.1, 5.3
+// With tasks of more than 10 blocks a lane, where a chain of rounds ends the call, U =
+// 2 loses: lognormal rows FP64 108 (U = 4) against 121, FP32 81 (6) against 89; 16
+// random columns a row, FP64, 49 against 61.  Nor do the next columns pay there: 12
+// random columns a row, FP32, 87 (kDenseValues, 6) against 106, lognormal 18 against 24.
+enum DenseLoads : int { kDenseColumns, kDenseValues, kDenseNext };
 constexpr int kDenseShort = 10;
+template <typename V> constexpr int kDenseAhead = sizeof(V) == 8 ? 4 : 6;
+template <typename V> constexpr int kDenseFew = sizeof(V) == 8 ? 3 : 6;
+template <typename V> constexpr DenseLoads kDenseFewLoads = sizeof(V) == 8 ? kDenseColumns : kDenseValues;
+template <typename V> constexpr int kDenseFewAhead = sizeof(V) == 8 ? 4 : 2;
 
-template <typename V, int U>
+template <typename V, int U, DenseLoads LOADS>
 __global__ void __launch_bounds__(kWarpsPerBlock * 32)
 dense_block_kernel(const SlicedTask* __restrict__ tasks, long long num_tasks, const V* __restrict__ val,
                    const int32_t* __restrict__ col, const int32_t* __restrict__ rowid, const V* x, int n_cols, V* y, V* chunk_sum) {
@@ -164,19 +176,31 @@ dense_block_kernel(const SlicedTask* __restrict__ tasks, long long num_tasks, co
   const V* vp = val + (size_t)(base + lane) * 4;
   const int32_t* cp = col + base + lane;
   V acc = V(0);
+  int next[U];
+  if constexpr (LOADS == kDenseNext) {
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (u < steps) next[u] = __ldcs(cp + u * 32);
+  }
   for (int k = 0; k < steps; k += U) {
     int c[U];
     V v[U][4];
 #pragma unroll
     for (int u = 0; u < U; ++u)
       if (k + u < steps) {
-        c[u] = __ldcs(cp + (k + u) * 32);
-        Quad<V>::load(vp + (size_t)(k + u) * 128, v[u]);
+        c[u] = LOADS == kDenseNext ? next[u] : __ldcs(cp + (k + u) * 32);
+        if constexpr (LOADS != kDenseColumns) Quad<V>::load(vp + (size_t)(k + u) * 128, v[u]);
       }
+    if constexpr (LOADS == kDenseNext) {
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        if (k + U + u < steps) next[u] = __ldcs(cp + (k + U + u) * 32);
+    }
 #pragma unroll
     for (int u = 0; u < U; ++u)
       if (k + u < steps) {
         V xv[4];
+        if constexpr (LOADS == kDenseColumns) Quad<V>::load(vp + (size_t)(k + u) * 128, v[u]);
 #pragma unroll
         for (int l = 0; l < 4; ++l) xv[l] = c[u] + l < n_cols ? ld_prev(x + c[u] + l) : V(0);
 #pragma unroll
@@ -432,7 +456,9 @@ bool launch_dense(const SlicedMatrix& m, const void* x, void* y, cudaStream_t s)
     set_error("dense blocks: too many tasks for one launch");
     return false;
   }
-  const auto kern = m.longest <= kDenseShort ? dense_block_kernel<V, 2> : dense_block_kernel<V, kDenseAhead<V>>;
+  const auto kern = m.longest <= kDenseFew<V> ? dense_block_kernel<V, kDenseFewAhead<V>, kDenseFewLoads<V>>
+                    : m.longest <= kDenseShort ? dense_block_kernel<V, 2, kDenseNext>
+                                               : dense_block_kernel<V, kDenseAhead<V>, kDenseValues>;
   return launch_chained(kern, (unsigned)grid, kWarpsPerBlock * 32, 0, s, m.tasks, m.num_tasks,
                         static_cast<const V*>(m.val), m.col, m.rowid, static_cast<const V*>(x), (int)m.n_cols,
                         static_cast<V*>(y), static_cast<V*>(m.chunk_sum));
