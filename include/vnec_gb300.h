@@ -472,8 +472,8 @@ typedef struct {
   int window_rows;     /* rows sorted by length within windows of this size (0: 65536) */
   int max_steps;       /* a row group spreads over enough slots to take at most this many steps (0: 32,
                           FP64 and DF32 16 for k <= 8 below 2^22 nonzeros) */
-  int unroll;          /* kernel mode: 1 normal load steps in flight per lane, 2 doubled, 3 each
-                          task's columns and values read in bulk (128 per round) and passed to
+  int unroll;          /* kernel mode: 1 normal load steps in flight per lane, 2 more of them (FP64:
+                          twice), 3 each task's columns and values read in bulk (128 per round) and passed to
                           the slots by shuffles; 0: tuned or normal */
   int host_parts;      /* host-vector calls run in this many parts so that X and Y copies overlap the
                           compute (0: 8, 1: one part) */

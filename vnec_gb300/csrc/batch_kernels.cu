@@ -37,7 +37,7 @@
 //   k =        2               8               32
 //   FP64   187 -> 103      304 -> 264      1063 -> 952   (122 -> 43)
 //   FP32   129 -> 74       142 -> 111       410 -> 301   (60 -> 41)
-//   DF32   168 -> 92       218 -> 174       643 -> 586   (94 -> 30)
+//   DF32   168 -> 91       218 -> 174       643 -> 587   (94 -> 31)
 
 #include <cuda_runtime.h>
 

@@ -249,8 +249,11 @@ SpB_VNEC_type IRD_VNEC(const SpB_Matrix A, SpB_Type type) {
 // with the same error bound, the handle used exactly like a merge-path one —
 // because the reference's harness sends every matrix of 3e6 rows or more to
 // VNEC-L (test_spmv_vnec.cpp:197,235-256), and at those sizes the merge-path
-// kernel is 2.5x slower than the selected plan on a power-law matrix (R-MAT
-// 2^24: 1.29 vs 0.91 ms).  A merge-path plan of any size stays available
+// kernel is 1.4x slower than the selected plan on a power-law matrix (R-MAT
+// 2^24: 1.28 vs 0.91 ms) and 1.8x on the 256^3 stencil (1.44 vs 0.78).  The line
+// was drawn on an earlier merge-path kernel; just below it the present one is
+// slower too (R-MAT 2^22: 4.9 against 3.5 ps a nonzero), but a caller that asks
+// for VNEC-L there gets it.  A merge-path plan of any size stays available
 // through SpB_VNEC_plan_ext with kernel SpB_VNEC_KERNEL_L.
 constexpr int64_t kBuildLSelectNnz = (int64_t)1 << 26;
 

@@ -8,8 +8,8 @@
 //   BF16 : values stored as BF16 (2 B) after scaling each row by a power of
 //          two (row exponent stored as int8), FP32 products/accumulation, the
 //          scale is applied exactly in FP64 after the FP64 lane reduction.
-//   DF32 : values stored as FP64 (8 B), split in-kernel into FP32 (hi, lo)
-//          pairs, x split once per call; Dekker products and TwoSum
+//   DF32 : values stored as FP32 (hi, lo) pairs (8 B), split at plan build, x
+//          split once per call (at the gather in small plans); Dekker products and TwoSum
 //          accumulation in FP32 (double-float), FP64 reductions — FP64-level
 //          accuracy on the FP32 pipe.  An x outside the split range raises a
 //          flag: the DF32 launch then returns at once and a guard launch of
