@@ -60,7 +60,7 @@ SpB_VNEC_type IRD_VNEC(const SpB_Matrix A, SpB_Type type);
  * plan of the automatic selection (the one SpB_mxv builds for a NULL handle),
  * because the reference's harness sends every matrix of 3e6 rows or more to
  * VNEC-L and the merge-path kernel is the slower plan at those sizes (R-MAT
- * 2^24: 1.29 vs 0.91 ms).  Either way SpMV_VNEC_L_* computes y := A x within
+ * 2^24: 1.28 vs 0.91 ms).  Either way SpMV_VNEC_L_* computes y := A x within
  * the same error bound; SpB_VNEC_plan_ext with kernel SpB_VNEC_KERNEL_L gives
  * a merge-path plan of any size.  The public fields num_merge_items and
  * items_per_thread are filled; the pointer fields are NULL.  Release with
