@@ -43,9 +43,10 @@ constexpr int kUnroll = 4;   // column entries in flight per lane
 // Blocks wanted in all: enough that a chunk with a hub column of tens of
 // thousands of entries is shared by many (half or twice as many: within 5%).
 constexpr long long kBlocks = 152LL * 16;
-// ... but no more than give each at least this many entries, were the frontier's
-// columns average and one the longest: every part scans its chunk anew (R-MAT
-// 2^13, dense x: 19.6 -> 13.5 us; 1,000 vertices of 2^18: 10.1 -> 8.3).
+// ... but beyond one block an SM no more than give each at least this many
+// entries, were the frontier's columns average and one the longest: every part
+// scans its chunk anew (R-MAT 2^13, dense x: 19.6 -> 13.5 us; fewer parts for
+// chunks that do not fill the GPU: 137 vertices of 2^16 9.2 -> 10.2).
 constexpr long long kPartEntries = 256;
 
 template <typename V>
@@ -181,8 +182,8 @@ bool launch(const PushMatrix& m, long long nx, const int32_t* idx, const void* x
   }
   const long long chunks = (nx + kChunk - 1) / kChunk;
   const long long most = kChunk * (m.nnz / std::max<long long>(m.n_cols, 1) + 1) + m.longest;
-  const long long parts =
-      std::max<long long>(1, std::min<long long>({kBlocks / chunks, 64, (most + kPartEntries - 1) / kPartEntries}));
+  const long long want = std::max<long long>(152 / chunks, (most + kPartEntries - 1) / kPartEntries);
+  const long long parts = std::max<long long>(1, std::min<long long>({kBlocks / chunks, 64, want}));
   if (chunks * parts > 0x7fffffffLL) {
     set_error("SpMSpV: too many entries of x for one launch");
     return false;

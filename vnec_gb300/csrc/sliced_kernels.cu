@@ -152,6 +152,9 @@ template <> struct Quad<float> {
 // random columns a row, FP32, 87 (kDenseValues, 6) against 106, lognormal 18 against 24.
 enum DenseLoads : int { kDenseColumns, kDenseValues, kDenseNext };
 constexpr int kDenseShort = 10;
+// Up to here kDenseNext; FP32 plans of 9 and 10 blocks keep kDenseValues (27-point
+// stencil 65^3 10.5 us against 12.3, 160^3 112 against 115; 9 random columns 24 and 23).
+template <typename V> constexpr int kDenseNextMost = sizeof(V) == 8 ? 10 : 8;
 template <typename V> constexpr int kDenseAhead = sizeof(V) == 8 ? 4 : 6;
 template <typename V> constexpr int kDenseFew = sizeof(V) == 8 ? 3 : 6;
 template <typename V> constexpr DenseLoads kDenseFewLoads = sizeof(V) == 8 ? kDenseColumns : kDenseValues;
@@ -457,7 +460,8 @@ bool launch_dense(const SlicedMatrix& m, const void* x, void* y, cudaStream_t s)
     return false;
   }
   const auto kern = m.longest <= kDenseFew<V> ? dense_block_kernel<V, kDenseFewAhead<V>, kDenseFewLoads<V>>
-                    : m.longest <= kDenseShort ? dense_block_kernel<V, 2, kDenseNext>
+                    : m.longest <= kDenseNextMost<V> ? dense_block_kernel<V, 2, kDenseNext>
+                    : m.longest <= kDenseShort ? dense_block_kernel<V, 2, kDenseValues>
                                                : dense_block_kernel<V, kDenseAhead<V>, kDenseValues>;
   return launch_chained(kern, (unsigned)grid, kWarpsPerBlock * 32, 0, s, m.tasks, m.num_tasks,
                         static_cast<const V*>(m.val), m.col, m.rowid, static_cast<const V*>(x), (int)m.n_cols,
